@@ -627,6 +627,7 @@ int lfgpu_solve(lfgpu_t h, const lfgpu_solve_options* o, double* u_out, lfgpu_re
         s.rhs = h->f;
         s.x = h->u;
         s.x0 = nullptr;
+        h->resident_ran = false;
         const bool had_bsr = h->bsr_version == h->k_version;
         float ms = 0.f;
         double apply_ms = 0.0;
@@ -699,7 +700,8 @@ int lfgpu_solve(lfgpu_t h, const lfgpu_solve_options* o, double* u_out, lfgpu_re
         r.storage_convert_ms = (blocks && !had_bsr && h->bsr_version == h->k_version) ? h->last_convert_ms : 0.0;
         r.matvec_calls = r.iterations + r.refinements;
         r.matrix_bytes_per_matvec =
-            blocks
+            h->resident_ran ? h->nnz / 4 * ((s.mixed ? 4 * 4 : 4 * 8) + 2)
+            : blocks
                 ? h->nblocks * (s.mixed ? 4 * 4 + (h->bcol16_ok ? 2 : 4) : 4 * 8 + 4)
                 : h->nnz * (s.mixed ? 4 + (h->col16_ok ? 2 : 4) : 8 + 4);
         // True residual ||f - K u|| in FP64.

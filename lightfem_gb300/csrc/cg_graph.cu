@@ -1,4 +1,7 @@
-// Preconditioned CG as a device-driven CUDA graph.
+// Preconditioned CG as a device-driven CUDA graph: the separately applied
+// preconditioners, the profiling form, and the pointwise preconditioners where the
+// resident kernel (cg_resident.cu) does not take the pattern (unpaired, or rows whose
+// columns span more nodes than a CTA's shared memory holds).
 //
 // Same recurrences as the persistent kernel in pcg.cu (pcg_solve,
 // src/solver.cpp:532-627, in FP64; the FP32-inner / FP64-refinement scheme in
@@ -26,6 +29,7 @@
 // FP64 loop runs its block solves between the update and the r.z reduction (as
 // IC(0) runs its sweeps), the mixed loop applies FP32 block inverses after each
 // iteration's IF node.
+#include "cg_math.cuh"
 #include "common.cuh"
 #include "kernels.hpp"
 
@@ -189,81 +193,6 @@ __device__ __forceinline__ bool reduce_last(const CgArgs& a, int slot, double (&
     __shared__ double s_red[32 * kMaxReduce];
     block_sum<K>(v, s_red);
     return reduce_tail<K>(a, slot, v, s_red, fin);
-}
-
-// An unevaluated FP32 pair (hi + lo) for the dot products of the FP32 loop: each
-// addition is Knuth's two-sum, so the pair carries about 48 bits.  This keeps
-// the dot products near FP64 accuracy with FP32 arithmetic only -- FP64 shuffles
-// and adds in every thread would keep GB300's narrow FP64 pipe busy for several
-// microseconds per reduction.
-struct FloatPair {
-    float hi = 0.f, lo = 0.f;
-    __device__ __forceinline__ void add(float x) {
-        const float s = __fadd_rn(hi, x);
-        const float bp = __fsub_rn(s, hi);
-        const float e = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(x, bp));
-        lo = __fadd_rn(lo, e);
-        hi = s;
-    }
-    __device__ __forceinline__ void add(const FloatPair& o) {
-        add(o.hi);
-        lo = __fadd_rn(lo, o.lo);
-    }
-};
-
-// FP32-pair per-thread values summed over the CTA (the mixed inner loop): warp
-// sums as pairs, then the warps' pairs in warp 0, whose threads all get the CTA's
-// totals as pairs in w (the other threads' w is zero).  FP32 arithmetic only: on
-// GB300 a dependent FP64 add takes about as long as a dozen FP32 ones.
-// NT > 0: only the CTA's first NT threads take part, synchronised on named barrier 1.
-template <int NT>
-__device__ __forceinline__ void pair_reduce_sync() {
-    if constexpr (NT == 0)
-        __syncthreads();
-    else
-        asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory");
-}
-
-template <int K, int NT = 0>
-__device__ __forceinline__ void block_pair_reduce(FloatPair (&v)[K], FloatPair (&w)[K]) {
-    __shared__ float2 s_warp[32 * kMaxReduce];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            FloatPair other;
-            other.hi = __shfl_xor_sync(0xffffffffu, v[k].hi, o);
-            other.lo = __shfl_xor_sync(0xffffffffu, v[k].lo, o);
-            v[k].add(other);
-        }
-    }
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) s_warp[warp * K + k] = make_float2(v[k].hi, v[k].lo);
-    }
-    pair_reduce_sync<NT>();
-#pragma unroll
-    for (int k = 0; k < K; ++k) w[k] = FloatPair{};
-    if (warp == 0) {
-        const int nw = (NT == 0 ? static_cast<int>(blockDim.x) : NT) >> 5;
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            if (lane < nw) {
-                const float2 t = s_warp[lane * K + k];
-                w[k].hi = t.x;
-                w[k].lo = t.y;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                FloatPair other;
-                other.hi = __shfl_xor_sync(0xffffffffu, w[k].hi, o);
-                other.lo = __shfl_xor_sync(0xffffffffu, w[k].lo, o);
-                w[k].add(other);
-            }
-        }
-    }
-    pair_reduce_sync<NT>();  // s_warp is free again
 }
 
 // The grid-wide step for FP32-pair values: each CTA leaves its pair totals, and
@@ -482,24 +411,6 @@ __device__ __forceinline__ void csr32_rows(const CgArgs& a, const G& g, Out&& ou
     });
 }
 
-__device__ __forceinline__ double2 block2_apply(const double* __restrict__ blk, int i, double r0, double r1) {
-    const double f0 = blk[3 * i], f1 = blk[3 * i + 1], f2 = blk[3 * i + 2];
-    double s0 = __dmul_rn(r0, f0);
-    double s1 = __dmul_rn(__dsub_rn(r1, __dmul_rn(f1, s0)), f2);
-    s1 = __dmul_rn(s1, f2);
-    s0 = __dmul_rn(__dsub_rn(s0, __dmul_rn(f1, s1)), f0);
-    return make_double2(s0, s1);
-}
-
-__device__ __forceinline__ float2 block2_apply32(const float* __restrict__ blk, int i, float r0, float r1) {
-    const float f0 = blk[3 * i], f1 = blk[3 * i + 1], f2 = blk[3 * i + 2];
-    float s0 = r0 * f0;
-    float s1 = (r1 - f1 * s0) * f2;
-    s1 = s1 * f2;
-    s0 = (s0 - f1 * s1) * f0;
-    return make_float2(s0, s1);
-}
-
 template <int PRECOND>
 __device__ __forceinline__ double2 precond64(const CgArgs& a, int i, double2 rv) {
     if (PRECOND == LFGPU_PRECOND_JACOBI) {
@@ -507,17 +418,6 @@ __device__ __forceinline__ double2 precond64(const CgArgs& a, int i, double2 rv)
         return make_double2(d.x * rv.x, d.y * rv.y);
     }
     return block2_apply(a.blk64, i, rv.x, rv.y);
-}
-
-// z of node i from the preconditioner's values pc (Jacobi: the inverse diagonal,
-// two floats a node; 2x2 blocks: the factor, three floats a node), wherever they are.
-template <int PRECOND>
-__device__ __forceinline__ float2 precond32_at(const float* pc, int i, float2 rv) {
-    if (PRECOND == LFGPU_PRECOND_JACOBI) {
-        const float2 d = reinterpret_cast<const float2*>(pc)[i];
-        return make_float2(d.x * rv.x, d.y * rv.y);
-    }
-    return block2_apply32(pc, i, rv.x, rv.y);
 }
 
 template <int PRECOND>
@@ -671,42 +571,8 @@ __global__ void __launch_bounds__(kThreads) cg64_direction(CgArgs a) {
 // last residual replacement is kept as an unevaluated FP32 pair (hi + lo, about
 // 48 significant bits) and added to the FP64 solution when a replacement is due,
 // so no FP64 arithmetic runs per iteration.
-__device__ __forceinline__ float pnew(float z, float p, float beta) { return __fmaf_rn(beta, p, z); }
-__device__ __forceinline__ float with_diag(float off, float hi, float lo, float x) { return fmaf(hi, x, off) + lo * x; }
-
 __device__ __forceinline__ float4* zp_buffer(const CgArgs& a, long long it) {
     return reinterpret_cast<float4*>((it & 1) ? a.zp1 : a.zp0);
-}
-
-// (hi, lo) += (ah + al) * p with error-free transformations (Knuth's two-sum,
-// the fma two-product), then renormalised so |lo| <= ulp(hi) / 2.  The _rn
-// intrinsics keep the compiler from fusing the steps the error terms rely on.
-__device__ __forceinline__ void pair_axpy(float& hi, float& lo, float ah, float al, float p) {
-    const float prod = __fmul_rn(ah, p);
-    const float perr = __fmaf_rn(al, p, __fmaf_rn(ah, p, -prod));
-    const float s = __fadd_rn(hi, prod);
-    const float bp = __fsub_rn(s, hi);
-    const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, bp)), __fsub_rn(prod, bp));
-    const float l = __fadd_rn(lo, __fadd_rn(err, perr));
-    hi = __fadd_rn(s, l);
-    lo = __fsub_rn(l, __fsub_rn(hi, s));
-}
-
-// num / den as an unevaluated FP32 pair (hi + lo, about 44 bits; Dekker's
-// division): one FP32 quotient, its remainder from an error-free product, and a
-// correction.  The loop's scalars (alpha, beta) come from this instead of an FP64
-// division, whose dependent steps take a large part of a microsecond on GB300
-// and hold up every CTA waiting for them.
-__device__ __forceinline__ void pair_quotient(double num, double den, float& hi, float& lo) {
-    const float nh = static_cast<float>(num), nl = static_cast<float>(num - static_cast<double>(nh));
-    const float dh = static_cast<float>(den), dl = static_cast<float>(den - static_cast<double>(dh));
-    const float q1 = __fdiv_rn(nh, dh);
-    const float p = __fmul_rn(q1, dh);
-    const float pe = __fmaf_rn(q1, dh, -p);  // q1 * dh = p + pe exactly
-    const float r = __fadd_rn(__fsub_rn(__fsub_rn(nh, p), pe), __fsub_rn(nl, __fmul_rn(q1, dl)));
-    const float q2 = __fdiv_rn(r, dh);
-    hi = __fadd_rn(q1, q2);
-    lo = __fsub_rn(q2, __fsub_rn(hi, q1));
 }
 
 // Preconditioners applied by their own kernels (the subdomain block solves,
@@ -2424,6 +2290,11 @@ PcgResult finish_cg(Context& c, const SolveSetup& s);
 PcgResult run_cg_graph(Context& c, const SolveSetup& s, float* kernel_ms) {
     const i64 n = c.n;
     LF_REQUIRE(n % 2 == 0, LFGPU_ERR_ARGUMENT, "the GPU PCG needs an even number of DOFs (u,v pairs)");
+    c.resident_ran = false;
+    if (s.unrolled == 0 && (s.precond == LFGPU_PRECOND_JACOBI || s.precond == LFGPU_PRECOND_BLOCK2)) {
+        PcgResult res{};
+        if (run_resident(c, s, &res, kernel_ms)) return res;
+    }
     const int blocks = c.num_sms * (2048 / kThreads);
     CgArgs a{};
     a.n = static_cast<int>(n);

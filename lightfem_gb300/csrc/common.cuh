@@ -203,6 +203,26 @@ struct Context {
     unsigned long long pattern_version = 0;
     std::vector<int> h_brow;
 
+    // The resident PCG's copy of K in slices of 32 nodes (cg_resident.cu): structure
+    // per pattern version, values per K version and precision.
+    struct Resident {
+        struct Grid {              // [0] FP64, [1] mixed: the launch's CTAs
+            Buf<int2> window;      // per CTA: the nodes its rows' columns span
+            int info[3] = {0, 0, 0};  // widest window, most blocks in a row, farthest column
+            unsigned long long version = ~0ull;
+        } grid[2];
+        bool uniform = true;       // one group of off-diagonal blocks in every slice
+        int groups = 0;
+        Buf<int> group_ptr, info;
+        Buf<uint4> off;
+        Buf<float4> v32, d32;
+        Buf<float2> dlo;
+        Buf<double2> v64, d64;
+        Buf<unsigned long long> words;  // packed sums
+        unsigned long long pattern_version = ~0ull, k_version[2] = {~0ull, ~0ull};
+    } resident;
+    bool resident_ran = false;  // the last solve ran there
+
     // IC(0) factor on the pattern of K (ic0.cu): left of the diagonal L(r, c), on
     // it the pivot, right of it L(c, r).  Built per K version; the mirror map (for
     // every upper entry, the index of its lower twin) per pattern version.

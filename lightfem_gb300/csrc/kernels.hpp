@@ -42,6 +42,10 @@ struct SolveSetup {
 };
 PcgResult run_pcg(Context& c, const SolveSetup& s, float* kernel_ms);
 
+// cg_resident.cu: the same solver for the pointwise preconditioners in one resident
+// kernel; false (nothing done) when the pattern is not one it takes
+bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms);
+
 // cg_graph.cu: the same solver as a device-driven CUDA graph of per-phase kernels
 PcgResult run_cg_graph(Context& c, const SolveSetup& s, float* kernel_ms);
 // FP64 PCG with a preconditioner applied by its own kernels inside the graph: the
