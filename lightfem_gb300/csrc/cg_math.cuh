@@ -133,9 +133,7 @@ __device__ __forceinline__ void pair_axpy(float& hi, float& lo, float ah, float 
 // correction.  The loop's scalars (alpha, beta) come from this instead of an FP64
 // division, whose dependent steps take a large part of a microsecond on GB300
 // and hold up every CTA waiting for them.
-__device__ __forceinline__ void pair_quotient(double num, double den, float& hi, float& lo) {
-    const float nh = static_cast<float>(num), nl = static_cast<float>(num - static_cast<double>(nh));
-    const float dh = static_cast<float>(den), dl = static_cast<float>(den - static_cast<double>(dh));
+__device__ __forceinline__ void pair_quotient(float nh, float nl, float dh, float dl, float& hi, float& lo) {
     const float q1 = __fdiv_rn(nh, dh);
     const float p = __fmul_rn(q1, dh);
     const float pe = __fmaf_rn(q1, dh, -p);  // q1 * dh = p + pe exactly
@@ -143,6 +141,11 @@ __device__ __forceinline__ void pair_quotient(double num, double den, float& hi,
     const float q2 = __fdiv_rn(r, dh);
     hi = __fadd_rn(q1, q2);
     lo = __fsub_rn(q2, __fsub_rn(hi, q1));
+}
+__device__ __forceinline__ void pair_quotient(double num, double den, float& hi, float& lo) {
+    const float nh = static_cast<float>(num), nl = static_cast<float>(num - static_cast<double>(nh));
+    const float dh = static_cast<float>(den), dl = static_cast<float>(den - static_cast<double>(dh));
+    pair_quotient(nh, nl, dh, dl, hi, lo);
 }
 
 }  // namespace

@@ -11,44 +11,54 @@
 // Layout.  K's 2x2 blocks lie in slices of 32 nodes, a thread per node: for each of
 // a node's eight off-diagonal blocks the slice holds 32 consecutive values, so a
 // warp's loads are whole lines, no lane is idle at a nine-block row, and no
-// shuffles are needed (on GB300 an FP64 instruction holds an SM's FP64 pipe for 19
-// cycles whatever its active lanes: the quarter-warp rows of cg64_product spent 72
-// of them a node, this form 36).  Neighbours are 16-bit offsets from the node.
+// shuffles are needed.  On GB300 an FP64 instruction holds its quarter of the SM for
+// 64 cycles (19 an SM over the four quarters) whatever its active lanes: the
+// quarter-warp rows of cg64_product spent 72 of them a node, this form 36.
+// Neighbours are 16-bit offsets from the node.
 //
 // p in shared memory.  A CTA owns consecutive slices; the columns of its rows span
 // a window of nodes, and the CTA keeps p of the whole window in shared memory.
-// z is what the CTAs exchange (through L2): each forms p = z + beta p for its
-// window, its neighbours' nodes included, with the same operation, so every copy
-// of a p is the same bit for bit and no third crossing publishes p.
+// z is what the CTAs exchange: each forms p = z + beta p for its window, its
+// neighbours' nodes included, with the same operation, so every copy of a p is the
+// same bit for bit and no third crossing publishes p.
 //
-// Sums.  A dot product's CTA totals are added as integers: with the previous
-// iteration's total as the scale, a total becomes an 88-bit fixed-point number
-// (2^-70 of the scale), whose two words are added to two counters in L2 by
-// red.add.  The top byte of a word counts the arrivals, so the poll that sees the
-// last CTA also has the sum, and the order of arrival does not matter.  A total
-// out of range, or a sum that lost more than ten bits of the scale, sends all CTAs
-// to a plain sum of the FP64 totals behind a counter.  152 CTAs, GB300: 0.83 us
-// without and 1.40 us with the release and acquire that publish z, against 2.6 us
-// for a counter and 152 FP64 partials.
+// Sums.  A thread's share of a dot product becomes a fixed-point number, scaled by the
+// previous iteration's total, in limbs that a warp adds with one instruction each and
+// a CTA in shared memory; a CTA's sum then travels in two words, added to two
+// counters in L2 by red.add.  The top byte of a word counts the arrivals, so the poll
+// that sees the last CTA also has the sum.  Integers: the order of arrival does not
+// matter, and the total is that of the shares to 2^-56 (FP32 pairs) or 2^-62 (FP64) of
+// the scale.  A share out of range, or a total that lost more than ten bits of the
+// scale, sends all CTAs to a plain sum of FP64 totals behind a counter.  A crossing of
+// 152 CTAs takes 0.83 us this way (1.40 us with a release and acquire that publish z),
+// against 2.6 us for a counter and 152 FP64 partials.
 //
-// Small meshes run in one thread-block cluster, whose CTAs exchange their totals
-// through distributed shared memory and a cluster barrier (0.2 us).
+// Three ways to meet.  kCluster, small meshes: one thread-block cluster; z and the
+// words go to the peers' shared memory with st.async and red.async, which count their
+// bytes on the receiver's mbarrier (0.25 us a crossing).  kTagged: the grid; z goes to
+// L2 in words that carry the iteration's number, so that it needs no fence and the
+// warps past the first fetch it while warp 0 waits for the sums.  kPublished, large
+// meshes: plain z behind release and acquire, half the bytes.
 //
 // Measured, us an iteration as a graph of kernels and here (n x n plane-strain
 // cantilevers, log-normal moduli, RCM, Jacobi; GB300):
-//   n            8     50    100   200   400   640   800   1000
-//   FP64  graph  28.5  29.8  32.1  36.1  57.7  ~97         200
-//         here    6.3   7.8   8.4  11.2  23.9  50.2  74.3  106
-//   mixed graph  20.9  20.0  20.1  21.5  24.5  ~33         58
-//         here    3.9   6.0   7.3   7.6  10.5  13.3  34.1  49.3
-// FP64 is bound by the FP64 pipe from 300 on (50 instructions a node, 39 us at 640);
-// mixed by the crossings up to 640 and by HBM from 800 on, where K leaves L2.
+//   n            8     20    50    80    100   200   300   400   500   640   800   1000
+//   FP64  graph  28.5        29.8        32.1  36.1  44.9  57.7        ~97         200
+//         here    4.8   4.9   5.6   6.0   7.2   8.5  14.2  22.0  29.8  48.7  74.3  106
+//   mixed graph  20.9        20.0        20.1  21.5  24.2  24.5   28   ~33         58
+//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.6   7.4   8.3  11.3  34.1  49.3
+// FP64 is bound by the FP64 pipe from 200 on (52 instructions a node, 40 us at 640);
+// mixed by the crossings up to 400 and by HBM from 800 on, where K leaves L2.  With FP64
+// shuffles and FP64 scalars in the sums a mixed iteration took 3.9 us at 8, 6.0 at 50
+// and 7.6 at 200, an FP64 one 6.3, 7.8 and 11.2.
 #include "cg_math.cuh"
 #include "common.cuh"
 #include "kernels.hpp"
 
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
+#include <type_traits>
 #include <vector>
 
 namespace lfgpu {
@@ -59,9 +69,7 @@ using u64 = unsigned long long;
 constexpr int kSlice = 32;       // nodes per slice, a thread each
 constexpr int kGroup = 8;        // off-diagonal blocks per node and group
 constexpr int kMaxCluster = 16;
-constexpr int kWords = 8;        // words of one packed sum (two per quantity)
-constexpr int kScaleBits = 70;   // fixed-point bits below the previous total's leading bit
-constexpr int kRangeBits = 87;   // |total| < 2^87 units
+constexpr int kStaticSmem64 = 12 * 1024, kStaticSmem32 = 20 * 1024;  // beside the dynamic shared memory
 
 struct ResArgs {
     int nb, slices, grid;
@@ -80,13 +88,15 @@ struct ResArgs {
     const double* x0;
     double* x;
     const void* pc;              // inverse diagonal or 2x2 factors, in the working precision
-    void* z;                     // published M^-1 r
+    void* z;                     // published M^-1 r (kTagged: as tagged words)
     void* r;                     // residual and product, where shared memory has no room for them
     void* q;
     float2* xhi;
     float2* xlo;
     int window_cap;              // nodes of the window in shared memory
+    int halo_cap;                // nodes of the arriving halo
     int own_cap;                 // nodes whose r and q are in shared memory (0: in global memory)
+    int x_cap;                   // the same for the solution or its correction pair
     int keep;                    // slices below this stay in L2, later ones stream
     u64* words;
     double* partials;
@@ -106,31 +116,38 @@ __device__ __forceinline__ u64 policy_keep() {
     return p;
 }
 // Matrix data: cached in L1 (CACHED: the CTA's share fits) or past it, with an L2 policy.
+// Volatile: a row's loads are issued together, before its arithmetic.
 template <bool CACHED>
 __device__ __forceinline__ float4 ld_matrix(const float4* p, u64 pol) {
-    if constexpr (CACHED) return __ldg(p);
     float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(p), "l"(pol));
+    if constexpr (CACHED)
+        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    else
+        asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                     : "l"(p), "l"(pol));
     return v;
 }
 template <bool CACHED>
 __device__ __forceinline__ double2 ld_matrix(const double2* p, u64 pol) {
-    if constexpr (CACHED) return __ldg(p);
     double2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
-                 : "=d"(v.x), "=d"(v.y)
-                 : "l"(p), "l"(pol));
+    if constexpr (CACHED)
+        asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+    else
+        asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.f64 {%0, %1}, [%2], %3;"
+                     : "=d"(v.x), "=d"(v.y)
+                     : "l"(p), "l"(pol));
     return v;
 }
 template <bool CACHED>
 __device__ __forceinline__ uint4 ld_matrix(const uint4* p, u64 pol) {
-    if constexpr (CACHED) return __ldg(p);
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p), "l"(pol));
+    if constexpr (CACHED)
+        asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    else
+        asm volatile("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "l"(p), "l"(pol));
     return v;
 }
 __device__ __forceinline__ int offset_of(const uint4& o, int k) {
@@ -139,15 +156,88 @@ __device__ __forceinline__ int offset_of(const uint4& o, int k) {
 }
 
 // ------------------------------------------------------------------ sums
+enum { kCluster = 0, kTagged = 1, kPublished = 2 };  // how the CTAs meet and exchange z
+enum { kGo = 0, kStop = 1, kRefine = 2 };
+enum { kPq = 0, kRr = 1, kRz = 2 };
+
+// A dot product's total: FP64, or an unevaluated FP32 pair in the mixed loop, whose
+// scalars then need no FP64 arithmetic.
+struct PairTotal {
+    float hi, lo;
+};
+template <bool MIXED>
+using Total = typename std::conditional<MIXED, PairTotal, double>::type;
+// Comparisons on the bits: an FP64 instruction takes 64 cycles.
+__device__ __forceinline__ long long bits_of(double v) { return __double_as_longlong(v); }
+__device__ __forceinline__ bool positive(double v) { return bits_of(v) > 0 && bits_of(v) < 0x7ff0000000000000ll; }
+__device__ __forceinline__ bool positive(PairTotal v) { return v.hi > 0.f && v.hi < INFINITY; }
+__device__ __forceinline__ void assign(double& t, double v) { t = v; }
+__device__ __forceinline__ void assign(PairTotal& t, double v) {
+    t.hi = static_cast<float>(v);
+    t.lo = static_cast<float>(v - static_cast<double>(t.hi));
+}
+// num / den of positive pairs as a pair of about 44 bits: a quotient by the
+// approximate reciprocal, its exact remainder, and a correction.
+__device__ __forceinline__ void quotient(PairTotal num, PairTotal den, float& hi, float& lo) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(den.hi));
+    if (!(den.hi > 0x1p-120f && den.hi < 0x1p120f)) {  // the approximate reciprocal's range
+        pair_quotient(num.hi, num.lo, den.hi, den.lo, hi, lo);
+        return;
+    }
+    const float q1 = __fmul_rn(num.hi, y);
+    const float r = __fadd_rn(__fmaf_rn(-q1, den.hi, num.hi), __fmaf_rn(-q1, den.lo, num.lo));
+    const float q2 = __fmul_rn(r, y);
+    hi = __fadd_rn(q1, q2);
+    lo = __fsub_rn(q2, __fsub_rn(hi, q1));
+}
+
+// Fixed point.  A share of a sum is cut into limbs of 21 bits (FP32 pairs: three, in
+// units of 2^-15, 2^-36 and 2^-56 of the scale 2^e) or 22 bits (FP64: four, in units
+// of 2^-70, 2^-48, 2^-26 and 2^-4), each a 32-bit integer that a warp adds with one
+// instruction; 1024 threads' limbs do not overflow.
+template <bool MIXED>
+constexpr int kLimbs = MIXED ? 3 : 4;
+constexpr int kScaleBits = 70;   // FP64: bits below the scale
+constexpr int kNoScale = 1 << 20;
+// Exponent of a positive normal total with room for the arithmetic around it, or kNoScale.
+__device__ __forceinline__ int exponent_of(double v) {
+    const int e = static_cast<int>(static_cast<u64>(bits_of(v)) >> 52);  // the sign counts too
+    return e > 123 && e < 1923 ? e - 1023 : kNoScale;
+}
+__device__ __forceinline__ int exponent_of(PairTotal v) {
+    const int e = static_cast<int>(__float_as_uint(v.hi) >> 23);
+    return e > 0 && e < 250 ? e - 127 : kNoScale;
+}
+
 struct ResShared {
-    double total[3];             // last totals: p.q, r.r, r.z
+    int e[3];                    // scales of the sums: exponents of the last totals (p.q, r.r, r.z)
+    float up[3], down[3][2];     // mixed: 2^-e, and 2^(e - 36) as a product of two floats
+    int limb[2][4];              // the CTA's sums being formed
+    int bad;                     // a thread's share was out of range
+    int next;                    // kGo, kStop, kRefine
+    int state;                   // of the last sum: 0 a wait ran out, 1 done, 2 to be formed in FP64
+    int fail;                    // a wait for a neighbour's z ran out
+    int peers;
     double alpha64, beta64;
     float alpha, alpha_lo, beta;
-    int next;                    // kGo, kStop, kRefine
-    int ok;
-    double xch[2][2][kMaxCluster];  // cluster: the peers' totals
+    u64 acc[2][4];               // cluster: the totals' words, added by the peers
+    double xch[2][2][kMaxCluster];  // cluster: the peers' FP64 totals
+    u64 mbar[4];                 // cluster: fixed-point sums 0 and 1, FP64 sums 0 and 1
+    int4 peer[kMaxCluster];      // cluster: first and end of this CTA's nodes in a peer's window, place there, rank
 };
-enum { kGo = 0, kStop = 1, kRefine = 2 };
+
+__device__ __forceinline__ void set_scale(ResShared& sh, int k, double t) { sh.e[k] = exponent_of(t); }
+__device__ __forceinline__ void set_scale(ResShared& sh, int k, PairTotal t) {
+    const int e = exponent_of(t);
+    sh.e[k] = e;
+    if (e != kNoScale) {  // e in [-126, 122]
+        sh.up[k] = __int_as_float((127 - e) << 23);
+        const int n = e - 36, a = n >> 1;
+        sh.down[k][0] = __int_as_float((a + 127) << 23);
+        sh.down[k][1] = __int_as_float((n - a + 127) << 23);
+    }
+}
 
 __device__ __forceinline__ u64 ld_relaxed(const u64* p) {
     u64 v;
@@ -165,16 +255,14 @@ __device__ __forceinline__ void red_add(u64* p, u64 v) {
     else asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Spin until done(value) holds; bounded by the handle's wait limit, and ended by
+// Spin until read() returns true; bounded by the handle's wait limit, and ended by
 // another CTA's abort.
-template <bool PUBLISH, typename Done>
-__device__ __forceinline__ bool spin(const u64* p, u64& v, DeviceStatus* status, u64 limit, Done&& done) {
-    v = PUBLISH ? ld_acquire(p) : ld_relaxed(p);
-    if (done(v)) return true;
+template <typename Read>
+__device__ __forceinline__ bool spin(DeviceStatus* status, u64 limit, Read&& read) {
+    if (read()) return true;
     const u64 t0 = global_ns();
     for (unsigned it = 1;; ++it) {
-        v = PUBLISH ? ld_acquire(p) : ld_relaxed(p);
-        if (done(v)) return true;
+        if (read()) return true;
         if (global_ns() - t0 > limit) {
             atomicExch(&status->abort, 1u);
             record_failure(status, LFGPU_ERR_TIMEOUT, static_cast<int>(blockIdx.x));
@@ -184,10 +272,172 @@ __device__ __forceinline__ bool spin(const u64* p, u64& v, DeviceStatus* status,
     }
 }
 
-// The grid's sum of K values, one per CTA, by warp 0 of every CTA (v: in all its
-// lanes, totals on return).  `prev`: the scale, last sums of the same quantities;
-// buf: the packed sum's words, next: words that CTA 0 clears for later sums when
-// this one publishes (their last readers arrived before this CTA got here).
+// The limbs of a thread's share; false when it is out of range.  FP32 pair: each limb
+// is the remainder so far rounded to the limb's unit, by adding 1.5 x 2^23, and the
+// remainders are exact.  |share| < 2^5 of the scale.
+__device__ __forceinline__ bool to_limbs(const ResShared& sh, int k, const FloatPair& v, int (&l)[3]) {
+    constexpr float kRound = 12582912.f;
+    constexpr int kBits = 0x4b400000;
+    const float hi = __fmul_rn(v.hi, sh.up[k]), lo = __fmul_rn(v.lo, sh.up[k]);
+    const float a = __fmaf_rn(hi, 0x1p15f, kRound);
+    const float r = __fmaf_rn(__fsub_rn(a, kRound), -0x1p-15f, hi);
+    const float b = __fmaf_rn(r, 0x1p36f, kRound), c = __fmaf_rn(lo, 0x1p36f, kRound);
+    const float s = __fmaf_rn(__fsub_rn(b, kRound), -0x1p-36f, r), t = __fmaf_rn(__fsub_rn(c, kRound), -0x1p-36f, lo);
+    l[2] = __float_as_int(a) - kBits;
+    l[1] = (__float_as_int(b) - kBits) + (__float_as_int(c) - kBits);
+    l[0] = __float_as_int(__fmaf_rn(__fadd_rn(s, t), 0x1p56f, kRound)) - kBits;
+    return fabsf(hi) < 0x1p5f && fabsf(lo) < 0x1p-17f;
+}
+// FP64: the mantissa shifted to its place in units of 2^-70 of the scale.  |share| <
+// 2^17 of the scale.
+__device__ __forceinline__ bool to_limbs(const ResShared& sh, int k, double v, int (&l)[4]) {
+    const u64 b = static_cast<u64>(bits_of(v));
+    const int ex = static_cast<int>((b >> 52) & 0x7ff);
+    const u64 m = (b & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
+    const int n = max(ex, 1) - 1075 + kScaleBits - sh.e[k];
+    const bool ok = ex != 0x7ff && (m == 0 || n <= 34);
+    const int up = min(max(n, 0), 34), dn = min(max(-n, 0), 63);
+    const u64 lo = dn > 0 ? (m + (1ull << (dn - 1))) >> dn : m << up;
+    const u64 hi = up > 0 ? m >> (64 - up) : 0ull;
+    constexpr unsigned mask = 0x3fffffu;
+    const int l0 = static_cast<int>(static_cast<unsigned>(lo) & mask);
+    const int l1 = static_cast<int>(static_cast<unsigned>(lo >> 22) & mask);
+    const int l2 = static_cast<int>((static_cast<unsigned>(lo >> 44) | (static_cast<unsigned>(hi) << 20)) & mask);
+    const int l3 = static_cast<int>(hi >> 2);
+    const int sign = static_cast<int>(static_cast<long long>(b) >> 63);  // 0 or -1
+    l[0] = (l0 ^ sign) - sign;
+    l[1] = (l1 ^ sign) - sign;
+    l[2] = (l2 ^ sign) - sign;
+    l[3] = (l3 ^ sign) - sign;
+    return ok;
+}
+
+// A CTA's sum of a quantity travels in two words, low and high (a sector holds the four
+// words of r.r and r.z): arrivals in the top byte, CTAs out of range in the next, and
+// below them 40 bits of the sum, or the rest plus 2^39; 48 bits hold 255 CTAs' shares.
+// Units: 2^-56 of the scale (pairs), 2^-62 (FP64, rounded from the threads' 2^-70).
+constexpr long long kHighBias = 1ll << 39;
+constexpr long long kLowMask = (1ll << 40) - 1;
+template <bool MIXED>
+__device__ __forceinline__ u64 sum_word(const int* l, bool high, bool bad) {
+    long long lo, hi;
+    if (MIXED) {
+        lo = static_cast<long long>(l[0]) + (static_cast<long long>(l[1]) << 20) + (static_cast<long long>(l[2]) << 41);
+        hi = 0;
+    } else {
+        hi = static_cast<long long>(l[2]) + (static_cast<long long>(l[3]) << 22);  // units of 2^44
+        lo = (static_cast<long long>(l[0]) + (static_cast<long long>(l[1]) << 22) + 128) >> 8;
+        lo += (hi & 15) << 36;
+        hi >>= 4;
+    }
+    hi += lo >> 40;
+    lo &= kLowMask;
+    bad = bad || hi >= kHighBias || hi < -kHighBias;
+    return (1ull << 56) | (bad ? 1ull << 48 : 0ull) | (high ? (bad ? 0ull : static_cast<u64>(hi + kHighBias)) : static_cast<u64>(lo));
+}
+
+// A quantity's total from its two words' sums over n CTAs (low in even lanes, high in
+// odd ones), in both lanes; false when it is not positive and within ten bits of the
+// scale (then it is formed in FP64).
+__device__ __forceinline__ void halves(u64 word, int n, long long& lo, long long& hi) {
+    const u64 other = __shfl_xor_sync(0xffffffffu, word, 1);
+    const bool odd = threadIdx.x & 1;
+    lo = static_cast<long long>((odd ? other : word) & 0xffffffffffffull);
+    hi = static_cast<long long>((odd ? word : other) & 0xffffffffffffull) - n * kHighBias;
+}
+__device__ __forceinline__ bool from_words(const ResShared& sh, int k, u64 word, int n, PairTotal& out) {
+    long long lo, hi;
+    halves(word, n, lo, hi);
+    const bool ok = hi > -(1ll << 20) && hi < (1ll << 20);
+    const long long s = (hi << 40) + lo;  // units of 2^-56
+    // Parts of 20 or 21 bits, exact in FP32; their sum as a pair in units of 2^-36.
+    const float f2 = static_cast<float>(static_cast<int>(s >> 41));
+    const float f1 = static_cast<float>(static_cast<int>(s >> 20) & 0x1fffff);
+    const float f0 = static_cast<float>(static_cast<int>(s) & 0xfffff);
+    const float h = __fmaf_rn(f2, 0x1p21f, f1);
+    const float l = __fmaf_rn(f0, 0x1p-20f, __fadd_rn(__fmaf_rn(f2, 0x1p21f, -h), f1));
+    out.hi = __fmul_rn(__fmul_rn(h, sh.down[k][0]), sh.down[k][1]);
+    out.lo = __fmul_rn(__fmul_rn(l, sh.down[k][0]), sh.down[k][1]);
+    return ok && s >= (1ll << 46);
+}
+__device__ __forceinline__ bool from_words(const ResShared& sh, int k, u64 word, int n, double& out) {
+    long long lo, hi;
+    halves(word, n, lo, hi);
+    hi += lo >> 40;
+    lo &= kLowMask;
+    const bool ok = hi >= (1ll << 12) && hi < (1ll << 45);
+    const int lead = __clzll(hi);  // 19 to 51
+    const u64 w = (static_cast<u64>(hi) << lead) | ((static_cast<u64>(lo) << 24) >> ((64 - lead) & 63));
+    const u64 m = (w >> 11) + ((w >> 10) & 1);  // 53 bits, rounded
+    out = __longlong_as_double((static_cast<long long>(1023 + 41 - lead + sh.e[k] - 1) << 52) + static_cast<long long>(m));
+    return ok;
+}
+
+// Per-thread values to the CTA's totals in FP64, in all lanes of warp 0.
+template <int K>
+__device__ __forceinline__ void block_total(const double (&t)[K], double (&v)[K], double* s_red) {
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
+#pragma unroll
+    for (int k = 0; k < K; ++k) s_red[k * T + tid] = t[k];
+    __syncthreads();
+    if (tid < 32) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = 0.0;
+            for (int w = lane; w < T; w += 32) v[k] += s_red[k * T + w];
+            v[k] = warp_sum(v[k]);
+        }
+    }
+}
+template <int K>
+__device__ __forceinline__ void block_total(FloatPair (&t)[K], double (&v)[K], double*) {
+    FloatPair w[K];
+    block_pair_reduce<K>(t, w);
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = static_cast<double>(w[k].hi) + static_cast<double>(w[k].lo);
+}
+
+// ------------------------------------------------------------------ cluster
+__device__ __forceinline__ unsigned cluster_rank() {
+    unsigned r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Address of a shared-memory variable in CTA `rank` of the cluster.
+__device__ __forceinline__ unsigned peer_address(const void* p, unsigned rank) {
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+// Stores and additions to a peer's shared memory that count their bytes on its mbarrier.
+__device__ __forceinline__ void send(unsigned addr, double v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send(unsigned addr, float2 v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send(unsigned addr, double2 v, unsigned bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "d"(v.x), "d"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void send_add(unsigned addr, u64 v, unsigned bar) {
+    asm volatile("red.async.relaxed.cluster.shared::cluster.mbarrier::complete_tx::bytes.add.u64 [%0], %1, [%2];" ::"r"(addr),
+                 "l"(v), "r"(bar)
+                 : "memory");
+}
+
+// What a CTA needs to form sums with the others: the words of the packed sums (kSets
+// sets for p.q, as many for r.r and r.z), the FP64 sum's slots and counter; in a
+// cluster the phases of its mbarriers.
+constexpr int kSets = 4, kSetStride = 16;
 struct GridSync {
     u64* words;
     double* partials;
@@ -196,20 +446,23 @@ struct GridSync {
     u64 limit;
     int grid;
     u64 arrivals;                // of the counter, so far
+    unsigned phase;              // bit b: parity of the phase mbarrier b is in
 
+    // The grid's sums of K FP64 values by warp 0 of every CTA (v: in all its lanes).
+    // The CTAs' earlier writes are visible to all after it.
     template <int K>
     __device__ __forceinline__ bool plain(double (&v)[K]) {
         const int lane = threadIdx.x & 31;
         double* slot = partials + ((arrivals / grid) & 1) * static_cast<size_t>(grid) * kMaxReduce;
         arrivals += grid;
         int ok = 1;
+        __syncwarp();
         if (lane == 0) {
 #pragma unroll
             for (int k = 0; k < K; ++k) __stcg(slot + blockIdx.x * kMaxReduce + k, v[k]);
             red_add<true>(bar, 1ull);
-            u64 seen;
             const u64 want = arrivals;
-            ok = spin<true>(bar, seen, status, limit, [&](u64 s) { return s >= want; });
+            ok = spin(status, limit, [&] { return ld_acquire(bar) >= want; });
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
         __syncwarp();
@@ -223,185 +476,166 @@ struct GridSync {
         return true;
     }
 
-    template <int K, bool PUBLISH>
-    __device__ __forceinline__ bool sum(double (&v)[K], const double* prev, u64* buf, u64* next_a, u64* next_b) {
+    // A lane's word added over the CTAs (live lanes: 2 k and 2 k + 1).
+    // Words: the set's, and the ones CTA 0 clears for two iterations on.  Their last
+    // readers are past them, and CTA 0 sees the old values before it arrives at
+    // another sum, so nobody adds to a word before it is cleared.
+    template <bool PUBLISH>
+    __device__ __forceinline__ bool packed(u64& word, bool live, u64* set, u64* clear) {
         const int lane = threadIdx.x & 31;
-        if (PUBLISH && blockIdx.x == 0 && lane < kWords) {
-            asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(next_a + lane), "l"(0ull) : "memory");
-            asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(next_b + lane), "l"(0ull) : "memory");
+        u64 old = 0;
+        int ok = 1;
+        const u64 n = static_cast<u64>(grid);
+        if (clear != nullptr && blockIdx.x == 0 && lane >= 8 && lane < 14) {
+            // Two words of a p.q set, four of an r.r and r.z set.
+            u64* w = lane < 10 ? clear + (lane - 8) : clear + kSets * kSetStride + (lane - 10);
+            asm volatile("atom.relaxed.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(w), "l"(0ull) : "memory");
         }
+        if (live) {
+            red_add<PUBLISH>(set + lane, word);
+            ok = spin(status, limit, [&] {
+                word = PUBLISH ? ld_acquire(set + lane) : ld_relaxed(set + lane);
+                return (word >> 56) == n;
+            });
+        }
+        ok = ok && (old >> 56) != 255ull;  // never 255: waits for the exchange's answer
+        return __all_sync(0xffffffffu, ok) != 0;
+    }
+
+    // Cluster: wait for mbarrier b's phase, in which `bytes` arrive.
+    __device__ __forceinline__ bool arrive_and_wait(ResShared& sh, int b, unsigned bytes) {
+        if ((threadIdx.x & 31) == 0) mbar_expect_tx(sh.mbar + b, bytes);
         __syncwarp();
-        // The scale's exponent; the same in every CTA.
-        bool usable = true;
-        int e[K];
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const u64 b = static_cast<u64>(__double_as_longlong(prev[k]));
-            e[k] = static_cast<int>(b >> 52) - 1023;  // a negative value or NaN gives a large exponent
-            usable = usable && e[k] > -900 && e[k] < 900;
-        }
-        if (usable) {
-            const int k = min(lane >> 1, K - 1);
-            double mine = v[0];
-            int scale = e[0];
-            if (K > 1 && k == 1) {
-                mine = v[K - 1];
-                scale = e[K - 1];
-            }
-            const u64 b = static_cast<u64>(__double_as_longlong(mine));
-            const int ex = static_cast<int>((b >> 52) & 0x7ff);
-            const u64 m = (b & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
-            const int sh = (ex ? ex : 1) - 1075 + kScaleBits - scale;
-            const bool bad = ex == 0x7ff || (m != 0 && sh > kRangeBits - 53);
-            unsigned __int128 u = 0;
-            if (!bad) {
-                if (sh >= 0) u = static_cast<unsigned __int128>(m) << min(sh, kRangeBits - 53);
-                else if (sh > -54) u = (m + (1ull << (-sh - 1))) >> -sh;
-                if (b >> 63) u = static_cast<unsigned __int128>(0) - u;
-                u += static_cast<unsigned __int128>(1) << kRangeBits;
-            }
-            const u64 low = static_cast<u64>(u) & 0xffffffffffffull;
-            const u64 high = static_cast<u64>(u >> 48) & 0xffffffffffull;
-            const bool is_high = lane & 1;
-            u64 got = 0;
-            int ok = 1;
-            if (lane < 2 * K) {
-                red_add<PUBLISH>(buf + lane, (1ull << 56) | (is_high ? (bad ? 1ull << 48 : 0ull) | high : low));
-                const u64 n = static_cast<u64>(grid);
-                ok = spin<PUBLISH>(buf + lane, got, status, limit, [&](u64 s) { return (s >> 56) == n; });
-            }
-            if (!__all_sync(0xffffffffu, ok)) return false;
-            got &= (1ull << 56) - 1;
-            bool lost = false;
-            double t[K];
-#pragma unroll
-            for (int j = 0; j < K; ++j) {
-                const u64 lo = __shfl_sync(0xffffffffu, got, 2 * j), hi = __shfl_sync(0xffffffffu, got, 2 * j + 1);
-                const unsigned __int128 all = (static_cast<unsigned __int128>(hi & 0xffffffffffffull) << 48) + lo;
-                const __int128 s = static_cast<__int128>(
-                    all - (static_cast<unsigned __int128>(static_cast<unsigned>(grid)) << kRangeBits));
-                // Positive, and within ten bits of the scale: else the plain sum.
-                lost = lost || (hi >> 48) != 0 || s < (static_cast<__int128>(1) << (kScaleBits - 10));
-                const u64 top = static_cast<u64>(s >> 32);  // at least 28 bits, at most 64
-                const u64 rest = static_cast<u64>(s) & 0xffffffffull;
-                const int lead = __clzll(static_cast<long long>(top));
-                const u64 w = (top << lead) | (lead >= 32 ? rest << (lead - 32) : rest >> (32 - lead));
-                const double d = __ull2double_rn(w);  // s = w 2^(32 - lead), to 64 bits
-                t[j] = d * __longlong_as_double(static_cast<long long>(1023 + 32 - lead + e[j] - kScaleBits) << 52);
-            }
-            if (!lost) {
-#pragma unroll
-                for (int j = 0; j < K; ++j) v[j] = t[j];
-                return true;
-            }
-        }
-        return plain<K>(v);
+        const unsigned parity = (phase >> b) & 1u;
+        const bool ok = spin(status, limit, [&] { return mbar_try_wait(sh.mbar + b, parity); });
+        phase ^= 1u << b;
+        return __all_sync(0xffffffffu, ok) != 0;
     }
 };
 
-// Per-thread values to the CTA's totals, in all lanes of warp 0.
-template <int K>
-__device__ __forceinline__ void block_total(const double (&t)[K], double (&v)[K], double* s_red) {
-    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31;
-    if (T > 32) {
-        // Through shared memory: shuffles in every warp would hold the FP64 pipe
-        // 19 cycles per warp and step.
+// The sum over all CTAs of K per-thread values of quantities FIRST.., then
+// fin(totals) on thread 0 of every CTA; false when a wait ran out.  FAST: in fixed
+// point at the scales of the last totals, where they allow it.  PUBLISH (grid): the
+// CTAs' earlier global writes are visible to all after it.  halo_bytes (cluster): z
+// that the peers send for this sum.  it: the iteration, for the words' set.
+// meanwhile(): work of the warps past the first while warp 0 waits.  Consecutive sums
+// use different slots: a peer that is one sum ahead then cannot reach this one's.
+template <int SYNC, bool MIXED, int FIRST, int K, bool PUBLISH, bool FAST, typename V, typename Meanwhile, typename Fin>
+__device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync& g, double* s_red, V (&t)[K],
+                                       unsigned it, [[maybe_unused]] unsigned halo_bytes, Meanwhile&& meanwhile, Fin&& fin) {
+    const int lane = threadIdx.x & 31;
+    constexpr int kSlot = FIRST == kPq ? 0 : 1;
+    bool fast = FAST;
+    if (FAST) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) s_red[k * T + tid] = t[k];
-        __syncthreads();
-    } else {
-        __syncwarp();
+        for (int k = 0; k < K; ++k) fast = fast && sh.e[FIRST + k] != kNoScale;
     }
-    if (tid < 32) {
+    Total<MIXED> tot[K];
+    if (FAST && fast) {
+        constexpr int L = kLimbs<MIXED>;
+        int l[K][L];
+        bool in_range = true;
+#pragma unroll
+        for (int k = 0; k < K; ++k) in_range = to_limbs(sh, FIRST + k, t[k], l[k]) && in_range;
+        if (!in_range) sh.bad = 1;
 #pragma unroll
         for (int k = 0; k < K; ++k) {
-            double a = t[k], b = 0.0;
-            if (T > 32) {
-                a = s_red[k * T + lane];
-                int w = lane + 32;
-                for (; w + 32 < T; w += 64) {
-                    b += s_red[k * T + w];
-                    a += s_red[k * T + w + 32];
-                }
-                if (w < T) b += s_red[k * T + w];
+            int mine = 0;
+#pragma unroll
+            for (int j = 0; j < L; ++j) {
+                const int s = __reduce_add_sync(0xffffffffu, l[k][j]);
+                if (lane == j) mine = s;
             }
-            v[k] = a + b;
+            if (lane < L) atomicAdd(&sh.limb[k][lane], mine);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-            for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-        }
-    }
-}
-template <int K>
-__device__ __forceinline__ void block_total(FloatPair (&t)[K], double (&v)[K], double*) {
-    FloatPair w[K];
-    block_pair_reduce<K>(t, w);
-#pragma unroll
-    for (int k = 0; k < K; ++k) v[k] = static_cast<double>(w[k].hi) + static_cast<double>(w[k].lo);
-}
-
-__device__ __forceinline__ unsigned cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void store_peer(const double* slot, unsigned rank, double v) {
-    unsigned addr;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(slot)), "r"(rank));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-
-// The sum over all CTAs of K per-thread values, then fin(totals) on thread 0 of
-// every CTA; false when a wait ran out.  PUBLISH: the CTAs' earlier global writes
-// are visible to all after it.  FAST: the packed sum, scaled by prev.
-template <bool CLUSTER, int K, bool PUBLISH, bool FAST, typename V, typename Fin>
-__device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync& g, double* s_red, V (&t)[K],
-                                       const double* prev, unsigned parity, Fin&& fin) {
-    double v[K];
-    block_total<K>(t, v, s_red);
-    bool ok = true;
-    if constexpr (CLUSTER) {
-        const int lane = threadIdx.x & 31;
-        if (a.grid > 1) {
-            const unsigned rank = cluster_rank();
-            if (threadIdx.x < 32 && lane < a.grid) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) store_peer(&sh.xch[parity & 1][k][rank], lane, v[k]);
-            }
-            cluster_barrier();
-            if (threadIdx.x < 32) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) v[k] = lane < a.grid ? sh.xch[parity & 1][k][lane] : 0.0;
-#pragma unroll
-                for (int o = kMaxCluster / 2; o > 0; o >>= 1) {
-#pragma unroll
-                    for (int k = 0; k < K; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
-                }
-            }
-        }
-    } else {
+        __syncthreads();
         if (threadIdx.x < 32) {
-            // Two sets of words for the p.q sums (parity 0, 1), two for the others.
-            u64* base = a.words;
-            const unsigned it = parity >> 1;
-            u64* mine = base + (2 * (parity & 1) + (it & 1)) * 16;
-            if constexpr (FAST)
-                ok = g.sum<K, PUBLISH>(v, prev, mine, base + ((it + 1) & 1) * 16, base + (2 + ((it + 1) & 1)) * 16);
-            else
-                ok = g.plain<K>(v);
+            const bool live = lane < 2 * K;
+            const int k = K > 1 ? (lane >> 1) & 1 : 0;
+            const bool bad = sh.bad != 0;
+            u64 word = sum_word<MIXED>(sh.limb[k], lane & 1, bad);
+            __syncwarp();
+            if (lane < 8) (&sh.limb[0][0])[lane] = 0;
+            if (lane == 8) sh.bad = 0;
+            bool ok = true;
+            if constexpr (SYNC == kCluster) {
+                if (a.grid > 1) {
+                    // Lane: word lane & 3 to peers lane / 4, lane / 4 + 8.
+                    if ((lane & 3) < 2 * K)
+                        for (int p = lane >> 2; p < a.grid; p += 8)
+                            send_add(peer_address(&sh.acc[kSlot][lane & 3], p), word, peer_address(sh.mbar + kSlot, p));
+                    ok = g.arrive_and_wait(sh, kSlot, static_cast<unsigned>(a.grid * 2 * K * 8) + halo_bytes);
+                    word = sh.acc[kSlot][lane & 3];
+                    __syncwarp();
+                    if (live) sh.acc[kSlot][lane] = 0;
+                }
+            } else {
+                u64* set = a.words + ((FIRST == kPq ? 0 : kSets) + (it & (kSets - 1))) * kSetStride;
+                u64* clear = FIRST == kPq ? nullptr : a.words + ((it + 2) & (kSets - 1)) * kSetStride;
+                ok = g.packed<PUBLISH>(word, live, set, clear);
+            }
+            Total<MIXED> mt;
+            bool good = from_words(sh, FIRST + k, word, a.grid, mt);
+            good = good && ((word >> 48) & 0xff) == 0;
+            good = __all_sync(0xffffffffu, good || !live) != 0;
+            tot[0] = mt;
+            if constexpr (K > 1) {
+                if constexpr (MIXED) {
+                    tot[1].hi = __shfl_sync(0xffffffffu, mt.hi, 2);
+                    tot[1].lo = __shfl_sync(0xffffffffu, mt.lo, 2);
+                } else {
+                    tot[1] = __shfl_sync(0xffffffffu, mt, 2);
+                }
+            }
+            if (lane == 0) {
+                if (ok && good) fin(tot);
+                sh.state = !ok ? 0 : good ? 1 : 2;
+            }
+        } else {
+            if constexpr (SYNC != kCluster) meanwhile();
         }
+        __syncthreads();
+        const int state = sh.state;
+        if (state != 2) return state != 0 && sh.fail == 0;
+        if constexpr (SYNC == kCluster) halo_bytes = 0;  // z has arrived
     }
-    if (threadIdx.x == 0) {
-        if (ok) fin(v);
-        sh.ok = ok;
+    // In FP64, CTA by CTA.
+    double v[K];
+    bool ok = true;
+    block_total<K>(t, v, s_red);
+    if (threadIdx.x < 32) {
+        if constexpr (SYNC == kCluster) {
+            if (a.grid > 1) {
+                const unsigned rank = cluster_rank();
+                if (lane < a.grid) {
+                    const unsigned bar = peer_address(sh.mbar + 2 + kSlot, lane);
+#pragma unroll
+                    for (int k = 0; k < K; ++k) send(peer_address(&sh.xch[kSlot][k][rank], lane), v[k], bar);
+                }
+                ok = g.arrive_and_wait(sh, 2 + kSlot, static_cast<unsigned>(a.grid * K * 8) + halo_bytes);
+#pragma unroll
+                for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < a.grid ? sh.xch[kSlot][k][lane] : 0.0);
+            }
+        } else {
+            ok = g.plain<K>(v);
+        }
+        if (lane == 0) {
+            if (ok) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) assign(tot[k], v[k]);
+                fin(tot);
+            }
+            sh.state = ok;
+        }
     }
     __syncthreads();
-    return sh.ok != 0;
+    if constexpr (SYNC == kTagged) {
+        if (!(FAST && fast)) {  // not yet done above
+            if (threadIdx.x >= 32 && sh.state) meanwhile();
+            __syncthreads();
+        }
+    }
+    return sh.state != 0 && sh.fail == 0;
 }
 
 // ------------------------------------------------------------------ rows
@@ -508,45 +742,182 @@ __device__ __forceinline__ float2 to_working(double2 v, float2) {
 __device__ __forceinline__ double2 to_working(double2 v, double2) { return v; }
 
 // ------------------------------------------------------------------ the solver
-template <bool MIXED, int PRECOND, bool CLUSTER, bool CACHED>
-__global__ void __launch_bounds__(MIXED ? 1024 : 512, 1) resident_pcg(ResArgs a) {
+// A published z: two 64-bit words a value pair in FP32, four in FP64, each a 32-bit
+// part of a value over the publication's number, so that a reader sees from the
+// word itself whether it has arrived: no fence, and the wait for a neighbour's z
+// overlaps the wait for the sums.
+template <typename V>
+constexpr int kTagWords = sizeof(V) / 4;
+__device__ __forceinline__ void publish_tagged(u64* w, float2 v, unsigned tag) {
+    const u64 t = static_cast<u64>(tag) << 32;
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(w), "l"(t | __float_as_uint(v.x)),
+                 "l"(t | __float_as_uint(v.y))
+                 : "memory");
+}
+__device__ __forceinline__ void publish_tagged(u64* w, double2 v, unsigned tag) {
+    const u64 t = static_cast<u64>(tag) << 32;
+    const u64 x = static_cast<u64>(__double_as_longlong(v.x)), y = static_cast<u64>(__double_as_longlong(v.y));
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(w), "l"(t | (x >> 32)), "l"(t | (x & 0xffffffffull))
+                 : "memory");
+    asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(w + 2), "l"(t | (y >> 32)), "l"(t | (y & 0xffffffffull))
+                 : "memory");
+}
+__device__ __forceinline__ void ld_two(const u64* w, u64& a, u64& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(w) : "memory");
+}
+__device__ __forceinline__ bool read_tagged(const u64* w, unsigned tag, float2& v) {
+    u64 a, b;
+    ld_two(w, a, b);
+    v = make_float2(__uint_as_float(static_cast<unsigned>(a)), __uint_as_float(static_cast<unsigned>(b)));
+    return static_cast<unsigned>(a >> 32) == tag && static_cast<unsigned>(b >> 32) == tag;
+}
+__device__ __forceinline__ bool read_tagged(const u64* w, unsigned tag, double2& v) {
+    u64 a, b, c, d;
+    ld_two(w, a, b);
+    ld_two(w + 2, c, d);
+    v.x = __longlong_as_double(static_cast<long long>((a << 32) | (b & 0xffffffffull)));
+    v.y = __longlong_as_double(static_cast<long long>((c << 32) | (d & 0xffffffffull)));
+    return static_cast<unsigned>(a >> 32) == tag && static_cast<unsigned>(b >> 32) == tag &&
+           static_cast<unsigned>(c >> 32) == tag && static_cast<unsigned>(d >> 32) == tag;
+}
+
+// Threads of a CTA: 64 registers a thread let 32 warps stream the FP32 matrix; where it
+// sits in L1, and in FP64, which the FP64 pipe bounds, 16 warps with 128 registers do.
+constexpr int max_threads(bool mixed, bool cached) { return mixed && !cached ? 1024 : 512; }
+
+template <bool MIXED, int PRECOND, int SYNC, bool CACHED>
+__global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(ResArgs a) {
     using V = typename std::conditional<MIXED, float2, double2>::type;
     using Sum = typename std::conditional<MIXED, FloatPair, double>::type;
+    using Tot = Total<MIXED>;
+    constexpr bool kPublish = SYNC == kPublished;
     extern __shared__ __align__(16) unsigned char res_smem[];
     __shared__ ResShared sh;
-    __shared__ double s_red[MIXED ? 2 * 1024 : 2 * 512];
+    __shared__ double s_red[2 * max_threads(MIXED, CACHED)];
     const int tid = threadIdx.x, T = blockDim.x, warp = tid >> 5, W = T >> 5;
     const int cta = blockIdx.x;
     const int sb = static_cast<int>(static_cast<long long>(a.slices) * cta / a.grid);
     const int se = static_cast<int>(static_cast<long long>(a.slices) * (cta + 1) / a.grid);
+    const int n0 = min(a.nb, sb * kSlice), n1 = min(a.nb, se * kSlice);  // the CTA's nodes
     const int2 wnd = a.window[cta];
-    const int w0 = wnd.x, wn = wnd.y - wnd.x;
-    V* win = reinterpret_cast<V*>(res_smem);
-    V* const z = static_cast<V*>(a.z);
-    // r and q of the CTA's nodes, by place in the CTA.
-    V* const r = a.own_cap ? win + a.window_cap : static_cast<V*>(a.r) + sb * kSlice;
-    V* const q = a.own_cap ? r + a.own_cap : static_cast<V*>(a.q) + sb * kSlice;
+    const int w0 = wnd.x, left = n0 - wnd.x, halo = left + (wnd.y - n1);  // the window's other nodes
+    V* const win = reinterpret_cast<V*>(res_smem);
+    V* const own = win + left;                       // p of the CTA's nodes
+    V* const zh = win + a.window_cap;                // z of the halo as it arrives (not kPublished)
+    V* const state = zh + a.halo_cap;
+    // By place in the CTA: r; q, then z from the update to the next direction.
+    V* const r = a.own_cap ? state : static_cast<V*>(a.r) + sb * kSlice;
+    V* const q = a.own_cap ? state + a.own_cap : static_cast<V*>(a.q) + sb * kSlice;
+    // The solution: x (FP64) or the correction pair (mixed).
+    V* const xs = a.x_cap ? state + 2 * a.own_cap
+                          : MIXED ? reinterpret_cast<V*>(a.xhi) + sb * kSlice : reinterpret_cast<V*>(a.x) + sb * kSlice;
+    V* const xl = MIXED ? (a.x_cap ? xs + a.x_cap : reinterpret_cast<V*>(a.xlo) + sb * kSlice) : nullptr;
     const u64 pol_keep = policy_keep(), pol_stream = l2_evict_first_policy();
-    GridSync g{a.words, a.partials, a.bar, a.status, a.status->wait_limit_ns, a.grid, 0ull};
-    unsigned parity = 0;  // 2 * iterations + sums of this one: consecutive sums differ in the last bit
-    long long it = 0, refs = 0;
-    int status = 0, converged = 0, stagnated = 0;
-    double r0 = 0.0, rho = 0.0, rr_last = 0.0;  // kept by thread 0
-    double rmax = 0.0, rtrue = 0.0, rtrue_prev = 0.0;
-    int no_progress = 0;
-    if constexpr (CLUSTER) {
-        if (a.grid > 1) cluster_barrier();  // every CTA runs before a peer stores into it
-    }
-    auto each_node = [&](auto&& body) {  // this thread's nodes: body(slice, node, place)
+    GridSync g{a.words, a.partials, a.bar, a.status, a.status->wait_limit_ns, a.grid, 0ull, 0u};
+    unsigned it32 = 0;  // iterations, in every thread
+    unsigned tag = 0;   // publications of z
+    long long it = 0, refs = 0;  // from here on: kept by thread 0
+    int status = 0, converged = 0, stagnated = 0, no_progress = 0;
+    double r0 = 0.0, rtrue = 0.0, rtrue_prev = 0.0;
+    Tot rho{}, rr_last{};
+    // Mixed: squares of the inner residual norm, of its largest since the last replacement,
+    // and of the bounds on it.
+    float rr_max = 0.f;
+    const float refine_below = static_cast<float>(a.reduction * a.reduction);
+    const float stop_below = static_cast<float>(a.target * a.target);
+    // This thread's nodes: body(slice, node, place).
+    auto each_node = [&](auto&& body) {
         for (int s = sb + warp; s < se; s += W) {
             const int node = s * kSlice + (tid & 31);
             if (node < a.nb) body(s, node, node - sb * kSlice);
         }
     };
+    int reach_lo = 0, reach_hi = a.nb;  // nodes below reach_lo or from reach_hi on: in other CTAs' windows
+    if (tid == 0) {
+        sh.bad = sh.fail = 0;
+        sh.next = kGo;
+        for (int k = 0; k < 3; ++k) sh.e[k] = kNoScale;
+    }
+    if (tid < 8) {
+        (&sh.limb[0][0])[tid] = 0;
+        (&sh.acc[0][0])[tid] = 0;
+    }
+    if constexpr (SYNC == kCluster) {
+        if (tid == 0) {
+            for (int b = 0; b < 4; ++b) mbar_init(sh.mbar + b, 1);
+            mbar_init_fence();
+            // This CTA's nodes in the peers' windows: a peer's left halo starts its window,
+            // its right halo follows the left one.
+            int n = 0;
+            for (int p = 0; p < a.grid; ++p) {
+                const int2 pw = a.window[p];
+                const int p0 = min(a.nb, static_cast<int>(static_cast<long long>(a.slices) * p / a.grid) * kSlice);
+                const int p1 = min(a.nb, static_cast<int>(static_cast<long long>(a.slices) * (p + 1) / a.grid) * kSlice);
+                int4 e = make_int4(0, 0, 0, p);
+                if (p > cta) e = make_int4(max(n0, pw.x), min(n1, p0), -pw.x, p);
+                if (p < cta) e = make_int4(max(n0, p1), min(n1, pw.y), p0 - pw.x - p1, p);
+                if (e.x < e.y) sh.peer[n++] = e;
+            }
+            sh.peers = n;
+        }
+        __syncthreads();
+        if (a.grid > 1) cluster_barrier();  // every CTA runs, its mbarriers ready, before a peer sends to it
+    } else {
+        __shared__ int s_reach[2];
+        if (tid == 0) {
+            s_reach[0] = 0;
+            s_reach[1] = a.nb;
+        }
+        __syncthreads();
+        for (int c = tid; c < a.grid; c += T) {
+            const int2 pw = a.window[c];
+            if (c < cta) atomicMax(&s_reach[0], pw.y);
+            if (c > cta) atomicMin(&s_reach[1], pw.x);
+        }
+        __syncthreads();
+        reach_lo = s_reach[0];
+        reach_hi = s_reach[1];
+    }
+    // z of a node to whoever has it in a window; cluster: for the r.r and r.z sum in fixed
+    // point (mbarrier 1) or in FP64 (3).
+    int z_bar = 3;
+    const unsigned halo_bytes = static_cast<unsigned>(halo * static_cast<int>(sizeof(V)));
+    auto publish = [&](int node, V zv) {
+        if constexpr (SYNC == kCluster) {
+            const int peers = sh.peers;
+            for (int p = 0; p < peers; ++p) {
+                const int4 e = sh.peer[p];
+                if (node >= e.x && node < e.y)
+                    send(peer_address(zh + (node + e.z), e.w), zv, peer_address(sh.mbar + z_bar, e.w));
+            }
+        } else if (node < reach_lo || node >= reach_hi) {
+            if constexpr (SYNC == kTagged)
+                publish_tagged(static_cast<u64*>(a.z) + static_cast<size_t>(node) * kTagWords<V>, zv, tag);
+            else
+                __stcg(static_cast<V*>(a.z) + node, zv);
+        }
+    };
+    // z of the halo, by the warps past the first, while warp 0 waits for the sums.
+    auto fetch = [&] {
+        if constexpr (SYNC == kTagged) {
+            bool ok = true;
+            for (int j = tid - 32; j < halo && ok; j += T - 32) {
+                const int node = j < left ? w0 + j : n1 + (j - left);
+                const u64* w = static_cast<const u64*>(a.z) + static_cast<size_t>(node) * kTagWords<V>;
+                V zv;
+                ok = spin(a.status, g.limit, [&] { return read_tagged(w, tag, zv); });
+                zh[j] = zv;
+            }
+            if (!ok) sh.fail = 1;
+        }
+    };
+    auto nothing = [] {};
 
+    auto solve = [&]() -> bool {
     // ---- start: x, r, z; r.r (FP64) and r.z
     {
         double t[2] = {0.0, 0.0};
+        tag += 1;
         each_node([&](int, int node, int at) {
             double2 xv = make_double2(0.0, 0.0), rv;
             if (a.x0) {
@@ -555,54 +926,64 @@ __global__ void __launch_bounds__(MIXED ? 1024 : 512, 1) resident_pcg(ResArgs a)
             } else {
                 rv = __ldg(reinterpret_cast<const double2*>(a.f) + node);
             }
-            reinterpret_cast<double2*>(a.x)[node] = xv;
             const V rw = to_working(rv, V{});
             const V zv = precond_at<PRECOND>(a, node, rw);
             r[at] = rw;
-            __stcg(z + node, zv);
+            q[at] = zv;
+            own[at] = V{};
             if constexpr (MIXED) {
-                a.xhi[node] = make_float2(0.f, 0.f);
-                a.xlo[node] = make_float2(0.f, 0.f);
+                reinterpret_cast<double2*>(a.x)[node] = xv;
+                xs[at] = V{};
+                xl[at] = V{};
+            } else {
+                xs[at] = xv;
             }
+            publish(node, zv);
             t[0] += rv.x * rv.x + rv.y * rv.y;
             t[1] += static_cast<double>(rw.x * zv.x + rw.y * zv.y);
         });
-        for (int j = tid; j < wn; j += T) win[j] = V{};
-        const bool ok = reduce<CLUSTER, 2, true, false>(a, sh, g, s_red, t, nullptr, 1u, [&](const double* s) {
-            r0 = sqrt(fmax(0.0, s[0]));
-            rho = s[1];
-            rmax = rtrue = rtrue_prev = r0;
-            rr_last = s[0];
-            sh.total[0] = 0.0;
-            sh.total[1] = s[0];
-            sh.total[2] = s[1];
-            sh.beta = 0.f;
-            sh.beta64 = 0.0;
-            sh.next = kGo;
-            if (r0 <= a.target) {
-                converged = 1;
-                sh.next = kStop;
-            } else if (!(s[1] > 0.0) || !isfinite(s[1])) {
-                status = LFGPU_ERR_RHO_INITIAL;
-                sh.next = kStop;
-            }
-        });
-        if (!ok) return;
+        for (int j = tid; j < halo; j += T) win[j < left ? j : j + (n1 - n0)] = V{};
+        const bool ok = reduce<SYNC, false, kRr, 2, true, false>(
+            a, sh, g, s_red, t, 0u, halo_bytes, fetch, [&](const double* s) {
+                r0 = sqrt(fmax(0.0, s[0]));
+                assign(rho, s[1]);
+                assign(rr_last, s[0]);
+                rr_max = static_cast<float>(s[0]);
+                rtrue = rtrue_prev = r0;
+                Tot t0;
+                assign(t0, s[0]);
+                set_scale(sh, kRr, t0);
+                set_scale(sh, kRz, rho);
+                sh.beta = 0.f;
+                sh.beta64 = 0.0;
+                if (r0 <= a.target) {
+                    converged = 1;
+                    sh.next = kStop;
+                } else if (!(s[1] > 0.0) || !isfinite(s[1])) {
+                    status = LFGPU_ERR_RHO_INITIAL;
+                    sh.next = kStop;
+                }
+            });
+        if (!ok) return false;
     }
 
     while (sh.next != kStop) {
         // ---- p = z + beta p over the window
         if constexpr (MIXED) {
             const float beta = sh.beta;
-            for (int j = tid; j < wn; j += T) {
-                const float2 zv = __ldcg(z + w0 + j), pv = win[j];
-                win[j] = make_float2(pnew(zv.x, pv.x, beta), pnew(zv.y, pv.y, beta));
+            auto turn = [&](float2& p, float2 zv) { p = make_float2(pnew(zv.x, p.x, beta), pnew(zv.y, p.y, beta)); };
+            each_node([&](int, int, int at) { turn(own[at], q[at]); });
+            for (int j = tid; j < halo; j += T) {
+                const int place = j < left ? j : j + (n1 - n0);
+                turn(win[place], kPublish ? __ldcg(static_cast<const V*>(a.z) + w0 + place) : zh[j]);
             }
         } else {
             const double beta = sh.beta64;
-            for (int j = tid; j < wn; j += T) {
-                const double2 zv = __ldcg(z + w0 + j), pv = win[j];
-                win[j] = make_double2(fma(beta, pv.x, zv.x), fma(beta, pv.y, zv.y));
+            auto turn = [&](double2& p, double2 zv) { p = make_double2(fma(beta, p.x, zv.x), fma(beta, p.y, zv.y)); };
+            each_node([&](int, int, int at) { turn(own[at], q[at]); });
+            for (int j = tid; j < halo; j += T) {
+                const int place = j < left ? j : j + (n1 - n0);
+                turn(win[place], kPublish ? __ldcg(static_cast<const V*>(a.z) + w0 + place) : zh[j]);
             }
         }
         __syncthreads();
@@ -610,91 +991,93 @@ __global__ void __launch_bounds__(MIXED ? 1024 : 512, 1) resident_pcg(ResArgs a)
         {
             Sum t[1] = {};
             each_node([&](int s, int node, int at) {
-                const int wi = node - w0;
-                const V y = slice_row<CACHED>(a, s, node, win, wi, s < a.keep ? pol_keep : pol_stream);
-                const V p = win[wi];
+                const V y = slice_row<CACHED>(a, s, node, win, node - w0, s < a.keep ? pol_keep : pol_stream);
+                const V p = own[at];
                 q[at] = y;
                 if constexpr (MIXED) t[0].add(p.x * y.x + p.y * y.y);
                 else t[0] += p.x * y.x + p.y * y.y;
             });
-            const bool ok =
-                reduce<CLUSTER, 1, false, true>(a, sh, g, s_red, t, sh.total, parity++, [&](const double* s) {
-                    sh.total[0] = s[0];
-                    if (!(s[0] > 0.0) || !isfinite(s[0])) {
+            const bool ok = reduce<SYNC, MIXED, kPq, 1, false, true>(
+                a, sh, g, s_red, t, it32, 0u, nothing, [&](const Tot* s) {
+                    set_scale(sh, kPq, s[0]);
+                    if (!positive(s[0])) {
                         status = LFGPU_ERR_NOT_SPD;
                         sh.next = kStop;
                     } else if constexpr (MIXED) {
-                        pair_quotient(rho, s[0], sh.alpha, sh.alpha_lo);
+                        quotient(rho, s[0], sh.alpha, sh.alpha_lo);
                     } else {
                         sh.alpha64 = rho / s[0];
                     }
                 });
-            if (!ok) return;
+            if (!ok) return false;
         }
         if (sh.next == kStop) break;
         // ---- x += alpha p, r -= alpha q, z = M^-1 r; r.r and r.z
         {
             Sum t[2] = {};
+            tag += 1;
+            z_bar = sh.e[kRr] != kNoScale && sh.e[kRz] != kNoScale ? 1 : 3;
             if constexpr (MIXED) {
                 const float alpha = sh.alpha, alpha_lo = sh.alpha_lo;
                 each_node([&](int, int node, int at) {
-                    const float2 p = win[node - w0], qv = q[at];
-                    float2 rv = r[at], hv = a.xhi[node], lv = a.xlo[node];
-                    pair_axpy(hv.x, lv.x, alpha, alpha_lo, p.x);
-                    pair_axpy(hv.y, lv.y, alpha, alpha_lo, p.y);
+                    const float2 p = own[at], qv = q[at];
+                    float2 rv = r[at], hv = xs[at], lv = xl[at];
                     rv.x -= alpha * qv.x;
                     rv.y -= alpha * qv.y;
                     const float2 zv = precond_at<PRECOND>(a, node, rv);
-                    a.xhi[node] = hv;
-                    a.xlo[node] = lv;
+                    publish(node, zv);
                     r[at] = rv;
-                    __stcg(z + node, zv);
+                    q[at] = zv;
+                    pair_axpy(hv.x, lv.x, alpha, alpha_lo, p.x);
+                    pair_axpy(hv.y, lv.y, alpha, alpha_lo, p.y);
+                    xs[at] = hv;
+                    xl[at] = lv;
                     t[0].add(rv.x * rv.x + rv.y * rv.y);
                     t[1].add(rv.x * zv.x + rv.y * zv.y);
                 });
             } else {
                 const double alpha = sh.alpha64;
-                double2* x2 = reinterpret_cast<double2*>(a.x);
                 each_node([&](int, int node, int at) {
-                    const double2 p = win[node - w0], qv = q[at];
-                    double2 rv = r[at], xv = x2[node];
-                    xv.x += alpha * p.x;
-                    xv.y += alpha * p.y;
+                    const double2 p = own[at], qv = q[at];
+                    double2 rv = r[at], xv = xs[at];
                     rv.x -= alpha * qv.x;
                     rv.y -= alpha * qv.y;
                     const double2 zv = precond_at<PRECOND>(a, node, rv);
-                    x2[node] = xv;
+                    publish(node, zv);
                     r[at] = rv;
-                    __stcg(z + node, zv);
+                    q[at] = zv;
+                    xv.x += alpha * p.x;
+                    xv.y += alpha * p.y;
+                    xs[at] = xv;
                     t[0] += rv.x * rv.x + rv.y * rv.y;
                     t[1] += rv.x * zv.x + rv.y * zv.y;
                 });
             }
-            const bool ok =
-                reduce<CLUSTER, 2, true, true>(a, sh, g, s_red, t, sh.total + 1, parity++, [&](const double* s) {
-                    sh.total[1] = s[0];
-                    sh.total[2] = s[1];
+            const bool ok = reduce<SYNC, MIXED, kRr, 2, kPublish, true>(
+                a, sh, g, s_red, t, it32, halo_bytes, fetch, [&](const Tot* s) {
+                    set_scale(sh, kRr, s[0]);
+                    set_scale(sh, kRz, s[1]);
                     it += 1;
                     if constexpr (MIXED) {
                         // Only decides when to replace the residual: FP32 is enough.
-                        const double rn = static_cast<double>(__fsqrt_rn(static_cast<float>(fmax(0.0, s[0]))));
-                        rmax = fmax(rmax, rn);
-                        if (rn <= a.reduction * rmax || rn <= a.target || it >= a.maxit) {
+                        const float rr = fmaxf(0.f, s[0].hi);
+                        rr_max = fmaxf(rr_max, rr);
+                        if (rr <= refine_below * rr_max || rr <= stop_below || it >= a.maxit) {
                             sh.next = kRefine;
-                        } else if (!(s[1] > 0.0) || !isfinite(s[1])) {
+                        } else if (!positive(s[1])) {
                             status = LFGPU_ERR_RHO;
                             sh.next = kStop;
                         } else {
                             float lo;
-                            pair_quotient(s[1], rho, sh.beta, lo);
+                            quotient(s[1], rho, sh.beta, lo);
                             rho = s[1];
                         }
                     } else {
                         rr_last = s[0];
-                        if (fmax(0.0, s[0]) <= a.target2) {
+                        if (!(s[0] > a.target2)) {  // NaN counts as zero, as in the reference
                             converged = 1;
                             sh.next = kStop;
-                        } else if (!(s[1] > 0.0) || !isfinite(s[1])) {
+                        } else if (!positive(s[1])) {
                             status = LFGPU_ERR_RHO;
                             sh.next = kStop;
                         } else {
@@ -704,76 +1087,104 @@ __global__ void __launch_bounds__(MIXED ? 1024 : 512, 1) resident_pcg(ResArgs a)
                         }
                     }
                 });
-            if (!ok) return;
+            if (!ok) return false;
+            it32 += 1;
         }
         // ---- residual replacement: x += correction, r = f - K x in FP64, z, beta
         if constexpr (MIXED) {
             if (sh.next != kRefine) continue;
             double2* x2 = reinterpret_cast<double2*>(a.x);
-            each_node([&](int, int node, int) {
-                const float2 hv = a.xhi[node], lv = a.xlo[node];
+            each_node([&](int, int node, int at) {
+                const float2 hv = xs[at], lv = xl[at];
                 double2 xv = x2[node];
                 xv.x += static_cast<double>(hv.x) + static_cast<double>(lv.x);
                 xv.y += static_cast<double>(hv.y) + static_cast<double>(lv.y);
                 x2[node] = xv;
-                a.xhi[node] = make_float2(0.f, 0.f);
-                a.xlo[node] = make_float2(0.f, 0.f);
+                xs[at] = V{};
+                xl[at] = V{};
             });
             double none[1] = {0.0};
-            unsigned swap = parity;
-            if (!reduce<CLUSTER, 1, true, false>(a, sh, g, s_red, none, nullptr, swap++, [](const double*) {})) return;
+            if (!reduce<SYNC, false, kPq, 1, true, false>(a, sh, g, s_red, none, 0u, 0u, nothing, [](const double*) {}))
+                return false;
             double t[2] = {0.0, 0.0};
+            tag += 1;
+            z_bar = 3;
             each_node([&](int, int node, int at) {
                 const double2 rv = residual_row(a, node, a.x);
                 const float2 rw = to_working(rv, float2{});
                 const float2 zv = precond_at<PRECOND>(a, node, rw);
+                publish(node, zv);
                 r[at] = rw;
-                __stcg(z + node, zv);
+                q[at] = zv;
                 t[0] += rv.x * rv.x + rv.y * rv.y;
                 t[1] += static_cast<double>(rw.x * zv.x + rw.y * zv.y);
             });
-            const bool ok = reduce<CLUSTER, 2, true, false>(a, sh, g, s_red, t, nullptr, swap++, [&](const double* s) {
-                refs += 1;
-                sh.next = kGo;
-                const double rt = sqrt(fmax(0.0, s[0]));
-                rtrue = rt;
-                if (rt <= a.target) {
-                    converged = 1;
-                    sh.next = kStop;
-                } else if (refs >= a.max_ref || it >= a.maxit) {
-                    sh.next = kStop;
-                } else {
-                    no_progress = rt >= rtrue_prev ? no_progress + 1 : 0;
-                    if (no_progress >= 3) {
-                        stagnated = 1;
+            const bool ok = reduce<SYNC, false, kRr, 2, true, false>(
+                a, sh, g, s_red, t, 0u, halo_bytes, fetch, [&](const double* s) {
+                    refs += 1;
+                    sh.next = kGo;
+                    const double rt = sqrt(fmax(0.0, s[0]));
+                    rtrue = rt;
+                    if (rt <= a.target) {
+                        converged = 1;
                         sh.next = kStop;
-                    }
-                    rtrue_prev = fmin(rtrue_prev, rt);
-                    rmax = rt;
-                }
-                if (sh.next == kGo) {
-                    if (!(s[1] > 0.0) || !isfinite(s[1])) {
-                        status = LFGPU_ERR_RHO;
+                    } else if (refs >= a.max_ref || it >= a.maxit) {
                         sh.next = kStop;
                     } else {
-                        sh.beta = a.restart ? 0.f : static_cast<float>(s[1] / rho);
-                        rho = s[1];
-                        sh.total[1] = s[0];
-                        sh.total[2] = s[1];
+                        no_progress = rt >= rtrue_prev ? no_progress + 1 : 0;
+                        if (no_progress >= 3) {
+                            stagnated = 1;
+                            sh.next = kStop;
+                        }
+                        rtrue_prev = fmin(rtrue_prev, rt);
+                        rr_max = static_cast<float>(s[0]);
                     }
-                }
-            });
-            if (!ok) return;
+                    if (sh.next == kGo) {
+                        if (!(s[1] > 0.0) || !isfinite(s[1])) {
+                            status = LFGPU_ERR_RHO;
+                            sh.next = kStop;
+                        } else {
+                            const double last = static_cast<double>(rho.hi) + static_cast<double>(rho.lo);
+                            sh.beta = a.restart ? 0.f : static_cast<float>(s[1] / last);
+                            assign(rho, s[1]);
+                            Tot t0;
+                            assign(t0, s[0]);
+                            set_scale(sh, kRr, t0);
+                            set_scale(sh, kRz, rho);
+                        }
+                    }
+                });
+            if (!ok) return false;
         }
     }
-    if constexpr (MIXED) {
+    return true;
+    };
+    const bool solved = solve();
+    if constexpr (SYNC == kCluster) {
+        if (a.grid > 1) {
+            // No CTA leaves while a peer may still send to it.  After a wait that ran out
+            // sends may be on their way that no phase here tracks: 100 us for them.
+            cluster_barrier();
+            if (!solved) {
+                const u64 t0 = global_ns();
+                while (global_ns() - t0 < 100000ull) {
+                }
+            }
+        }
+    }
+    if (!solved) return;
+    {
         double2* x2 = reinterpret_cast<double2*>(a.x);
-        each_node([&](int, int node, int) {
-            const float2 hv = a.xhi[node], lv = a.xlo[node];
-            double2 xv = x2[node];
-            xv.x += static_cast<double>(hv.x) + static_cast<double>(lv.x);
-            xv.y += static_cast<double>(hv.y) + static_cast<double>(lv.y);
-            x2[node] = xv;
+        each_node([&](int, int node, int at) {
+            if constexpr (MIXED) {
+                const float2 hv = xs[at], lv = xl[at];
+                double2 xv = x2[node];
+                xv.x += static_cast<double>(hv.x) + static_cast<double>(lv.x);
+                xv.y += static_cast<double>(hv.y) + static_cast<double>(lv.y);
+                x2[node] = xv;
+            } else {
+                x2[node] = xs[at];
+            }
         });
     }
     if (cta == 0 && tid == 0) {
@@ -781,7 +1192,8 @@ __global__ void __launch_bounds__(MIXED ? 1024 : 512, 1) resident_pcg(ResArgs a)
         res.iterations = it;
         res.refinements = refs;
         res.initial_residual = r0;
-        res.final_residual = MIXED ? rtrue : sqrt(fmax(0.0, rr_last));
+        if constexpr (MIXED) res.final_residual = rtrue;
+        else res.final_residual = sqrt(fmax(0.0, rr_last));
         res.status = status;
         res.converged = converged;
         res.stagnated = stagnated;
@@ -824,6 +1236,7 @@ __global__ void __launch_bounds__(256) resident_windows(int nb, int slices, int 
         atomicMax(info + 0, s_hi - s_lo);
         atomicMax(info + 1, s_deg);
         atomicMax(info + 2, s_far);
+        atomicMax(info + 3, s_hi - s_lo - (n1 - n0));
     }
 }
 
@@ -933,31 +1346,29 @@ __global__ void resident_values(int nb, int slices, const int* __restrict__ grou
 
 // ------------------------------------------------------------------ launch shapes
 struct Shape {
-    bool cluster = false;
+    int sync = kPublished;
     int grid = 0, threads = 0, smem = 0;
-    int window_cap = 0, own_cap = 0;
+    int window_cap = 0, halo_cap = 0, own_cap = 0, x_cap = 0;
     bool cached = false;
 };
 
-// Meshes up to these many nodes run in one cluster.
+// Meshes up to these many nodes run in one cluster, up to these with tagged z.
 constexpr int kClusterNodes64 = 3600, kClusterNodes32 = 8192;
-constexpr int kStaticSmem64 = 12 * 1024, kStaticSmem32 = 20 * 1024;
+constexpr int kTaggedNodes64 = 300000, kTaggedNodes32 = 400000;
 
 int slices_of(const Context& c) { return static_cast<int>((c.n / 2 + kSlice - 1) / kSlice); }
 
 Shape launch_shape(const Context& c, bool mixed) {
     const int nodes = static_cast<int>(c.n / 2), slices = slices_of(c);
-    const int max_warps = mixed ? 32 : 16;
     Shape s;
-    s.cluster = nodes <= (mixed ? kClusterNodes32 : kClusterNodes64);
-    if (s.cluster) {
+    if (nodes <= (mixed ? kClusterNodes32 : kClusterNodes64)) {
+        s.sync = kCluster;
         s.grid = 1;
         while (s.grid < kMaxCluster && s.grid * (mixed ? 4 : 1) < slices) s.grid *= 2;
     } else {
+        s.sync = nodes <= (mixed ? kTaggedNodes32 : kTaggedNodes64) ? kTagged : kPublished;
         s.grid = c.num_sms;
     }
-    const int per = (slices + s.grid - 1) / s.grid;
-    s.threads = 32 * std::max(1, std::min(max_warps, per));
     return s;
 }
 
@@ -977,7 +1388,7 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
         resident_windows<<<s.grid, 256, 0, c.stream>>>(nb, slices, s.grid, c.rowptr, c.col, grid.window, res.info);
         LF_CUDA(cudaGetLastError());
         c.launches += 1;
-        LF_CUDA(cudaMemcpyAsync(grid.info, res.info.p, 3 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        LF_CUDA(cudaMemcpyAsync(grid.info, res.info.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, c.stream));
         LF_CUDA(cudaStreamSynchronize(c.stream));
         grid.version = c.pattern_version;
     }
@@ -985,15 +1396,27 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
     const int vec = mixed ? 8 : 16;
     int optin = 0;
     LF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
-    const int room = optin - (mixed ? kStaticSmem32 : kStaticSmem64);
+    const int room = (optin - (mixed ? kStaticSmem32 : kStaticSmem64)) / vec;
     s.window_cap = (grid.info[0] + 1) & ~1;
+    s.halo_cap = s.sync == kPublished ? 0 : (grid.info[3] + 1) & ~1;
     const int own = (slices + s.grid - 1) / s.grid * kSlice;
-    if (s.window_cap > room / vec) return false;
-    s.own_cap = (s.window_cap + 2 * own) <= room / vec ? own : 0;
-    s.smem = vec * (s.window_cap + 2 * s.own_cap);
+    int used = s.window_cap + s.halo_cap;
+    if (used > room) return false;
+    if (used + 2 * own <= room) {
+        s.own_cap = own;
+        used += 2 * own;
+        const int x = (mixed ? 2 : 1) * own;
+        if (used + x <= room) {
+            s.x_cap = own;
+            used += x;
+        }
+    }
+    s.smem = vec * used;
     // The CTA's matrix share fits L1 beside its shared memory.
-    const int row_bytes = mixed ? 8 * 16 + 16 + 16 + 8 + 24 : 8 * 32 + 32 + 16 + 48;
-    s.cached = s.cluster || own * row_bytes + s.smem < optin - 40 * 1024;
+    const int row_bytes = mixed ? 8 * 16 + 16 + 16 + 8 + 12 : 8 * 32 + 32 + 16 + 24;
+    s.cached = s.sync == kCluster || own * row_bytes + s.smem < optin - 24 * 1024;
+    s.threads = 32 * std::max(s.sync == kCluster ? 1 : 4,
+                              std::min(max_threads(mixed, s.cached) / 32, own / kSlice));
     if (res.pattern_version != c.pattern_version) {
         int groups = slices;
         res.uniform = grid.info[1] <= kGroup + 1;
@@ -1088,13 +1511,22 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
         a.q = c.v64[3].p;
     }
     a.window_cap = sh.window_cap;
+    a.halo_cap = sh.halo_cap;
     a.own_cap = sh.own_cap;
+    a.x_cap = sh.x_cap;
     a.keep = slices;
-    res.words.ensure(64);
+    if (sh.sync == kTagged) {
+        const size_t words = padded * (mixed ? kTagWords<float2> : kTagWords<double2>);
+        res.tagged.ensure(words);
+        LF_CUDA(cudaMemsetAsync(res.tagged.p, 0, words * sizeof(u64), c.stream));  // no tag of an earlier solve
+        a.z = res.tagged.p;
+    }
+    constexpr int kWordCount = 2 * kSets * kSetStride;
+    res.words.ensure(kWordCount);
     c.bar.ensure(1);
     c.partials.ensure(static_cast<size_t>(2) * sh.grid * kMaxReduce);
     c.pcg_result.ensure(1);
-    LF_CUDA(cudaMemsetAsync(res.words.p, 0, 64 * sizeof(u64), c.stream));
+    LF_CUDA(cudaMemsetAsync(res.words.p, 0, kWordCount * sizeof(u64), c.stream));
     LF_CUDA(cudaMemsetAsync(c.bar.p, 0, sizeof(u64), c.stream));
     LF_CUDA(cudaMemsetAsync(c.pcg_result.p, 0, sizeof(PcgResult), c.stream));
     a.words = res.words;
@@ -1114,7 +1546,9 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
     a.restart = s.restart;
     auto launch = [&](auto kernel) {
         LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem));
-        if (sh.cluster && sh.grid > 8)
+        LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     std::min(100, (sh.smem + kStaticSmem32) * 100 / (228 * 1024) + 1)));
+        if (sh.sync == kCluster && sh.grid > 8)
             LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(sh.grid);
@@ -1122,7 +1556,7 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
         cfg.dynamicSmemBytes = sh.smem;
         cfg.stream = c.stream;
         cudaLaunchAttribute attr[1] = {};
-        if (sh.cluster) {
+        if (sh.sync == kCluster) {
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = sh.grid;
             attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -1137,13 +1571,18 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
         LF_CUDA(cudaEventRecord(c.ev_b, c.stream));
         c.launches += 1;
     };
-    constexpr int J = LFGPU_PRECOND_JACOBI, B = LFGPU_PRECOND_BLOCK2;
-    if (mixed && sh.cluster) jac ? launch(resident_pcg<true, J, true, true>) : launch(resident_pcg<true, B, true, true>);
-    else if (mixed && sh.cached) jac ? launch(resident_pcg<true, J, false, true>) : launch(resident_pcg<true, B, false, true>);
-    else if (mixed) jac ? launch(resident_pcg<true, J, false, false>) : launch(resident_pcg<true, B, false, false>);
-    else if (sh.cluster) jac ? launch(resident_pcg<false, J, true, true>) : launch(resident_pcg<false, B, true, true>);
-    else if (sh.cached) jac ? launch(resident_pcg<false, J, false, true>) : launch(resident_pcg<false, B, false, true>);
-    else jac ? launch(resident_pcg<false, J, false, false>) : launch(resident_pcg<false, B, false, false>);
+    auto by_sync = [&](auto m, auto p) {
+        constexpr bool M = decltype(m)::value;
+        constexpr int P = decltype(p)::value;
+        if (sh.sync == kCluster) launch(resident_pcg<M, P, kCluster, true>);
+        else if (sh.sync == kTagged && sh.cached) launch(resident_pcg<M, P, kTagged, true>);
+        else if (sh.sync == kTagged) launch(resident_pcg<M, P, kTagged, false>);
+        else launch(resident_pcg<M, P, kPublished, false>);
+    };
+    using J = std::integral_constant<int, LFGPU_PRECOND_JACOBI>;
+    using B = std::integral_constant<int, LFGPU_PRECOND_BLOCK2>;
+    if (mixed) jac ? by_sync(std::true_type{}, J{}) : by_sync(std::true_type{}, B{});
+    else jac ? by_sync(std::false_type{}, J{}) : by_sync(std::false_type{}, B{});
     LF_CUDA(cudaMemcpyAsync(out, c.pcg_result.p, sizeof(PcgResult), cudaMemcpyDeviceToHost, c.stream));
     *kernel_ms = elapsed_ms(c);
     check_status(c);

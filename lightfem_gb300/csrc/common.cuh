@@ -208,7 +208,7 @@ struct Context {
     struct Resident {
         struct Grid {              // [0] FP64, [1] mixed: the launch's CTAs
             Buf<int2> window;      // per CTA: the nodes its rows' columns span
-            int info[3] = {0, 0, 0};  // widest window, most blocks in a row, farthest column
+            int info[4] = {0, 0, 0, 0};  // widest window, most blocks in a row, farthest column, widest halo
             unsigned long long version = ~0ull;
         } grid[2];
         bool uniform = true;       // one group of off-diagonal blocks in every slice
@@ -218,7 +218,8 @@ struct Context {
         Buf<float4> v32, d32;
         Buf<float2> dlo;
         Buf<double2> v64, d64;
-        Buf<unsigned long long> words;  // packed sums
+        Buf<unsigned long long> words;   // packed sums
+        Buf<unsigned long long> tagged;  // z as tagged words
         unsigned long long pattern_version = ~0ull, k_version[2] = {~0ull, ~0ull};
     } resident;
     bool resident_ran = false;  // the last solve ran there

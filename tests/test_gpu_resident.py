@@ -96,3 +96,17 @@ def test_iteration_cap(native):
         _, r = ctx.solve(ctx.options(1e-11, 7, "csr", "jacobi", precision))
         assert r.iterations == 7 and not r.converged
     ctx.close()
+
+
+@pytest.mark.parametrize("nx,ny", [(99, 101), (550, 540), (640, 630)])
+def test_exchanges_of_z(native, nx, ny):
+    """Past one cluster: z in tagged words (10,200 nodes), and published behind a release
+    (FP64 from 300,000 nodes, mixed from 400,000).  Both precisions agree to the FP64
+    stop rule's own accuracy on these meshes (1e-8, measured residuals of 1e-9)."""
+    model = indexed(grid(nx, ny))
+    ctx = system(native, model)
+    u, r = ctx.solve(ctx.options(1e-9, 50000, "csr", "jacobi"))
+    v, m = ctx.solve(ctx.options(1e-9, 50000, "bsr", "block", "mixed"))
+    assert r.converged and m.converged
+    assert np.linalg.norm(u - v) <= 1e-8 * np.linalg.norm(u)
+    ctx.close()
