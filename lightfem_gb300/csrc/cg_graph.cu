@@ -124,6 +124,7 @@ struct CgArgs {
     int product_grid;              // CTAs of mx_product (the direct form's update adds their p.q pairs)
     int sw_window;                 // ring slots per CTA (a power of two)
     int sw_maxp, sw_maxe;          // the largest piece: positions, entries (the stage size)
+    int pipe_warps, pipe_groups, pipe_stages;  // pipelined sweeps: warps a group, groups, stages
     void* sw_y;                    // forward result in backward positions (double or float)
     void* sw_rhs;                  // r in forward positions (double or float)
     float* sw_rr;                  // mixed: r32 in backward positions (the backward sweep's r.z)
@@ -1445,6 +1446,262 @@ __global__ void __cluster_dims__(kSweepCluster, 1, 1) __launch_bounds__(kSweepBl
     }
 }
 
+// ------------------------------------------------------------------ pipelined level sweeps
+// The same two sweeps by levels where no level holds more than kPipeMaxWidth rows, in
+// one CTA.  A level of the cluster's sweeps costs its rows' whole chain, nine FP64
+// products and nine differences of 64 cycles each, before the next may start.  But of
+// a row's terms only the last one to three need the level before it; the others'
+// operands are older.  Here the groups of warps take the levels in turn and work on
+// several at once: a warp forms its rows' terms in order, waiting for the third last
+// level before its own, the second last and the last only where its terms need them,
+// so that between levels only the last terms, the pivot's product and a trip through
+// shared memory are left.  The terms are subtracted in the same order as everywhere,
+// each rounded on its own: the result is the reference's bit for bit.  Consecutive
+// groups sit on different quarters of the SM (an FP64 instruction holds its quarter
+// for 64 cycles).
+//
+// Results go to a ring in shared memory; a warp done with a level arrives on the
+// level's mbarrier.  A level ends only after the one before it, so a wait covers all
+// earlier levels too, and kPipeDone mbarriers in turn are enough.  Operands come level
+// by level from the producer warps (cp.async.bulk) into stages; a stage is filled
+// again when the group's warps are done with it, so no warp is more levels ahead of
+// another than there are stages, and the ring spans the longest dependency and those
+// levels.
+//
+// What a level costs at 96x96 (FP64, RCM, up to 48 rows): 0.40 us; with a poll of each
+// operand or of a flag per warp in place of the mbarrier 0.77 and 0.43-0.50, with the
+// terms as predicated places in place of a loop 1.31 (an FP64 instruction holds its
+// quarter even where no lane is active), with one producer warp 0.60.  Bound by the
+// chain from level to level while levels are narrow, then by the FP64 pipe of one SM.
+//
+// us per application, forward and backward, before (polled in FP64, the cluster's
+// levels in a mixed iteration) and now (GB300, RCM cantilevers):
+//   rows in the widest level      6     49    126    151    201    251
+//   mesh                      10x10  96x96 250^2  300^2  400^2  500^2
+//   FP64 application     before  164   1772   5239   6866  10262  13951
+//                           now   68    616   2286   3031   4985   7613
+//   mixed iteration      before  141   1068   2752   3307   4435   5577
+//                           now   67    402   1391   1858   3192   5033
+// Wider levels stay with the cluster: eight SMs share a level's FP64 work and copies.
+// Bounded wait for a phase of this CTA's own mbarrier; the abort flag, a trip to L2, is
+// looked at rarely: the wait is on the way from level to level.
+__device__ __forceinline__ bool wait_own(unsigned long long* bar, unsigned parity, DeviceStatus* status, int level) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const unsigned long long t0 = global_ns();
+    for (unsigned it = 1;; ++it) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((it & 255u) == 0u && wait_expired(status, t0, level)) return false;
+    }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(32 * (kPipeWarps + kPipeProducers), 1) ic0_pipe_sweep(CgArgs a) {
+    using T = typename std::conditional<(MODE < 2), double, float>::type;
+    constexpr bool kFwd = (MODE & 1) == 0;
+    if (a.st->done) return;
+    extern __shared__ __align__(128) unsigned char pipe_smem[];
+    __shared__ __align__(8) unsigned long long full[kPipeStages], empty[kPipeStages], level_done[kPipeDone];
+    __shared__ int4 piece_of[kPipeStages];  // first and end position, first and end entry
+    __shared__ int4 since[kPipeStages];     // first positions of the third, second and last level before
+    __shared__ int s_failed, s_issued[kPipeProducers];
+    const CgArgs::SweepPlan& sp = a.sw[kFwd ? 0 : 1];
+    const int levels = sp.levels, S = a.pipe_stages, G = a.pipe_groups, GW = a.pipe_warps;
+    const int mask = a.sw_window - 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    T* ring = reinterpret_cast<T*>(pipe_smem);
+    unsigned char* stages = pipe_smem + static_cast<size_t>(a.sw_window) * sizeof(T);
+    const SweepStageLayout lay = sweep_stage_layout(static_cast<int>(sizeof(T)), a.sw_maxp, a.sw_maxe);
+    if (tid == 0) {
+        s_failed = 0;
+        for (int s = 0; s < S; ++s) {
+            mbar_init(full + s, 1);
+            mbar_init(empty + s, GW);
+        }
+        for (int s = 0; s < kPipeDone; ++s) mbar_init(level_done + s, GW);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    bool ok = true;
+    FloatPair rz;  // the mixed backward sweep's r.z
+    if (warp >= G * GW) {
+        // ---- producers: warp w copies the operands of levels w, w + kPipeProducers, ... into
+        // their stages.  The lanes read the bounds of the levels around one, a turn ahead.
+        const int w = warp - G * GW;
+        const unsigned long long policy = l2_evict_first_policy();
+        const T* rhs_src = static_cast<const T*>(kFwd ? a.sw_rhs : a.sw_y);
+        const int2* begin = reinterpret_cast<const int2*>(sp.level_begin);  // first position, first entry
+        // Lane i: the bounds of level L - 3 + i.
+        auto around = [&](int L) { return __ldg(begin + max(0, min(L - 3 + (lane & 7), levels))); };
+        int2 next = around(w);
+        int issued = w;  // past the last level issued
+        int s = w;       // the level's stage, L mod S, and the parity of the turn before
+        unsigned parity = 1;
+        for (int L = w; L < levels; L += kPipeProducers) {
+            const int2 cur = next;
+            next = around(L + kPipeProducers);
+            int4 before, pc;
+            before.x = __shfl_sync(0xffffffffu, cur.x, 0);
+            before.y = __shfl_sync(0xffffffffu, cur.x, 1);
+            before.z = __shfl_sync(0xffffffffu, cur.x, 2);
+            before.w = 0;
+            pc.x = __shfl_sync(0xffffffffu, cur.x, 3);
+            pc.y = __shfl_sync(0xffffffffu, cur.x, 4);
+            pc.z = __shfl_sync(0xffffffffu, cur.y, 3);
+            pc.w = __shfl_sync(0xffffffffu, cur.y, 4);
+            // After a wait that ran out nothing more is issued: a stage never holds more than
+            // one outstanding set of copies.
+            if (lane == 0 && ok && L >= S) ok = wait_own(empty + s, parity, a.status, L);
+            if (lane == 0 && ok) {
+                issued = L + kPipeProducers;
+                piece_of[s] = pc;
+                since[s] = before;
+                unsigned char* st = stages + static_cast<size_t>(s) * lay.bytes;
+                const int dep0 = pc.z - lead_of<int>(pc.z), val0 = pc.z - lead_of<T>(pc.z);
+                const int pos0 = pc.x - lead_of<T>(pc.x);
+                const bool entries = pc.w > pc.z;
+                const unsigned b_desc = static_cast<unsigned>(pc.y - pc.x) * 16u;
+                const unsigned b_dep = entries ? static_cast<unsigned>(sweep_round16((pc.w - dep0) * 4)) : 0u;
+                const unsigned b_val =
+                    entries ? static_cast<unsigned>(sweep_round16((pc.w - val0) * static_cast<int>(sizeof(T)))) : 0u;
+                const unsigned b_pos = static_cast<unsigned>(sweep_round16((pc.y - pos0) * static_cast<int>(sizeof(T))));
+                mbar_expect_tx(full + s, b_desc + b_dep + b_val + (MODE == 3 ? 3u : 2u) * b_pos);
+                bulk_copy(st + lay.desc, sp.desc + pc.x, b_desc, full + s, policy);
+                if (entries) {
+                    bulk_copy(st + lay.dep, sp.dep + dep0, b_dep, full + s, policy);
+                    bulk_copy(st + lay.val, static_cast<const T*>(sp.val) + val0, b_val, full + s, policy);
+                }
+                bulk_copy(st + lay.inv, static_cast<const T*>(sp.inv) + pos0, b_pos, full + s, policy);
+                bulk_copy(st + lay.rhs, rhs_src + pos0, b_pos, full + s, policy);
+                if (MODE == 3) bulk_copy(st + lay.rr, a.sw_rr + pos0, b_pos, full + s, policy);
+            }
+            __syncwarp();
+            s += kPipeProducers;
+            if (s >= S) {
+                s -= S;
+                parity ^= 1u;
+            }
+        }
+        if (lane == 0) s_issued[w] = issued;
+    } else {
+        // ---- consumers: group g takes levels g, g + G, ...; one row per thread.
+        const int group = warp / GW, at = (warp % GW) * 32 + lane;
+        float* zp_out = MODE == 3 ? reinterpret_cast<float*>(zp_buffer(a, a.st->it)) : nullptr;
+        // Wait until the group of level L is done with it (and so all levels before it);
+        // bounded.  After a wait that ran out a warp finishes its level with whatever the
+        // ring holds and takes no other.
+        auto wait_level = [&](int L) {
+            if (L >= 0 && ok)
+                ok = wait_own(level_done + L % kPipeDone, static_cast<unsigned>(L / kPipeDone) & 1u, a.status, L);
+        };
+        int s = group;  // the level's stage, L mod S, and the parity of its turn
+        unsigned parity = 0;
+        for (int L = group; L < levels; L += G) {
+            if (ok) ok = wait_own(full + s, parity, a.status, L);
+            ok = __all_sync(0xffffffffu, ok) != 0;
+            if (!ok) break;  // the stage may not have arrived
+            const int4 pc = piece_of[s], from = since[s];
+            const unsigned char* st = stages + static_cast<size_t>(s) * lay.bytes;
+            const int dep0 = pc.z - lead_of<int>(pc.z), val0 = pc.z - lead_of<T>(pc.z);
+            const int pos0 = pc.x - lead_of<T>(pc.x);
+            const int* sdep = reinterpret_cast<const int*>(st + lay.dep) - dep0;  // entry j at [j]
+            const T* sval = reinterpret_cast<const T*>(st + lay.val) - val0;
+            const bool have = at < pc.y - pc.x;
+            int4 d = make_int4(0, 0, 0, 0);
+            T acc = T(0), inv = T(0), rr = T(0);
+            // This row's first terms that need the third last, second last and last level.
+            int j3 = 0, j2 = 0, j1 = 0;
+            if (have) {
+                d = reinterpret_cast<const int4*>(st + lay.desc)[at];
+                acc = reinterpret_cast<const T*>(st + lay.rhs)[pc.x + at - pos0];
+                inv = reinterpret_cast<const T*>(st + lay.inv)[pc.x + at - pos0];
+                if constexpr (MODE == 3) rr = reinterpret_cast<const T*>(st + lay.rr)[pc.x + at - pos0];
+                j3 = j2 = j1 = d.z;
+                for (int j0 = d.z; j0 > d.y; j0 -= 6) {
+                    int p[6];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) p[k] = sdep[max(j0 - 1 - k, d.y)];
+#pragma unroll
+                    for (int k = 0; k < 6; ++k) {
+                        const int j = max(j0 - 1 - k, d.y);
+                        if (p[k] >= from.x) j3 = j;
+                        if (p[k] >= from.y) j2 = j;
+                        if (p[k] >= from.z) j1 = j;
+                    }
+                }
+            }
+            // Terms [j, end) of this row.  A loop, not predicated places: an FP64 instruction
+            // holds its quarter of the SM for 64 cycles even with no active lane.  The next
+            // term's operands are read while this one's product is formed.
+            auto terms = [&](int j, int end) {
+                if (j >= end) return;
+                T v = sval[j], x = ring[sdep[j] & mask];
+#pragma unroll 1
+                while (true) {
+                    const int n = min(j + 1, end - 1);
+                    const T t = sweep_mul(v, x);
+                    v = sval[n];
+                    x = ring[sdep[n] & mask];
+                    acc = sweep_sub(acc, t);
+                    if (++j >= end) break;
+                }
+            };
+            wait_level(L - 4);
+            terms(d.y, j3);
+            wait_level(L - 3);
+            terms(j3, j2);
+            wait_level(L - 2);
+            terms(j2, j1);
+            wait_level(L - 1);  // a level also ends after the one before it
+            terms(j1, d.z);
+            const T y = sweep_mul(acc, inv);
+            if (have) ring[(pc.x + at) & mask] = y;
+            __syncwarp();
+            if (lane == 0) {
+                arrive(level_done + L % kPipeDone);
+                arrive(empty + s);
+            }
+            if (have) {  // off the way to the next level
+                if constexpr (kFwd) {
+                    static_cast<T*>(a.sw_y)[d.w] = y;
+                } else if constexpr (MODE == 1) {
+                    a.z[d.x] = y;
+                } else {
+                    // z of DOF 2m sits in .x of node m's (z, p) float4, z of DOF 2m + 1 in .z.
+                    zp_out[4 * (d.x >> 1) + 2 * (d.x & 1)] = y;
+                    rz.add(rr * y);
+                }
+            }
+            s += G;
+            if (s >= S) {
+                s -= S;
+                parity ^= 1u;
+            }
+        }
+    }
+    if (!ok) s_failed = 1;
+    __syncthreads();
+    if (s_failed) {
+        // A wait ran out: end the solve (the status word says why).  Copies on their way
+        // land before this CTA releases its shared memory.
+        if (tid == 0) {
+            a.st->status = LFGPU_ERR_TIMEOUT;
+            a.st->done = 1;
+            set_loop(a, false);
+            for (int w = 0; w < kPipeProducers; ++w)  // each producer's last levels, one per stage
+                for (int L = s_issued[w] - kPipeProducers, k = 0; L >= 0 && k < S; L -= kPipeProducers, ++k) {
+                    if (!mbar_try_wait(full + L % S, static_cast<unsigned>(L / S) & 1u))
+                        mbar_drain(full + L % S, static_cast<unsigned>(L / S) & 1u);
+                }
+        }
+        __syncthreads();
+        return;
+    }
+    if constexpr (MODE == 3) {
+        FloatPair vv[1] = {rz};
+        reduce_last<1>(a, 2, vv, [&](const double* t) { rho_from_application(a, t); });
+    }
+}
+
 __device__ __forceinline__ void ic0_mark_pending(const CgArgs& a, int i) {
     if (a.y == nullptr) return;  // the subdomain preconditioner writes z without polls
     const double pending = __longlong_as_double(static_cast<long long>(kPending));
@@ -1950,6 +2207,9 @@ void build_fp64(cudaGraph_t g, CgArgs* a, int blocks) {
 
 constexpr int kBodyIterations = 8;
 
+// Threads of the pipelined IC(0) sweeps: the groups' warps and the producers.
+int pipe_threads(const CgArgs& a) { return 32 * (a.pipe_groups * a.pipe_warps + kPipeProducers); }
+
 // The mixed loop's separately applied preconditioners, after `dep`; returns the
 // last node.  Subdomain: one kernel (sub_grid CTAs of sub_threads); IC(0): the
 // forward and the backward FP32 level sweep (one cluster each, smem bytes of ring).
@@ -1963,6 +2223,11 @@ cudaGraphNode_t add_mixed_apply(cudaGraph_t g, cudaGraphNode_t dep, CgArgs* a, i
     } else {
         cudaGraphNode_t n0;
         add_kernel(g, &n0, &dep, 1, ic0_sweep_inputs<true>, a->blocks, a);
+        if (a->pipe_groups > 0) {
+            add_kernel(g, &n1, &n0, 1, ic0_pipe_sweep<2>, 1, a, smem, pipe_threads(*a));
+            add_kernel(g, &n2, &n1, 1, ic0_pipe_sweep<3>, 1, a, smem, pipe_threads(*a));
+            return n2;
+        }
         add_kernel(g, &n1, &n0, 1, ic0_level_sweep<2>, kSweepCluster, a, smem, kSweepBlock);
         add_kernel(g, &n2, &n1, 1, ic0_level_sweep<3>, kSweepCluster, a, smem, kSweepBlock);
         return n2;
@@ -2067,10 +2332,12 @@ void launch_unrolled(cudaStream_t stream, CgArgs* a, int blocks, bool mixed, int
         if constexpr (PRECOND == LFGPU_PRECOND_IC0) {
             ic0_sweep_inputs<true><<<a->blocks, kThreads, 0, stream>>>(*a);
             LF_CUDA(cudaGetLastError());
-            ic0_level_sweep<2><<<kSweepCluster, kSweepBlock, smem, stream>>>(*a);
+            if (a->pipe_groups > 0) ic0_pipe_sweep<2><<<1, pipe_threads(*a), smem, stream>>>(*a);
+            else ic0_level_sweep<2><<<kSweepCluster, kSweepBlock, smem, stream>>>(*a);
             LF_CUDA(cudaGetLastError());
             trail.mark(phase);
-            ic0_level_sweep<3><<<kSweepCluster, kSweepBlock, smem, stream>>>(*a);
+            if (a->pipe_groups > 0) ic0_pipe_sweep<3><<<1, pipe_threads(*a), smem, stream>>>(*a);
+            else ic0_level_sweep<3><<<kSweepCluster, kSweepBlock, smem, stream>>>(*a);
         } else {
             mx_sub_apply<<<sub_grid, sub_threads, 0, stream>>>(*a);
         }
@@ -2154,6 +2421,11 @@ cudaGraphNode_t add_apply(cudaGraph_t g, cudaGraphNode_t dep, CgArgs* a, const S
     if (ap.levels) {
         cudaGraphNode_t n0;
         add_kernel(g, &n0, &dep, 1, ic0_sweep_inputs<false>, a->blocks, a);
+        if (a->pipe_groups > 0) {
+            add_kernel(g, &n1, &n0, 1, ic0_pipe_sweep<0>, 1, a, ap.smem, pipe_threads(*a));
+            add_kernel(g, &n2, &n1, 1, ic0_pipe_sweep<1>, 1, a, ap.smem, pipe_threads(*a));
+            return n2;
+        }
         add_kernel(g, &n1, &n0, 1, ic0_level_sweep<0>, kSweepCluster, a, ap.smem, kSweepBlock);
         add_kernel(g, &n2, &n1, 1, ic0_level_sweep<1>, kSweepCluster, a, ap.smem, kSweepBlock);
         return n2;
@@ -2200,13 +2472,16 @@ void launch_separate_unrolled(cudaStream_t stream, CgArgs* a, int blocks, const 
         if (ap.levels) {
             ic0_sweep_inputs<false><<<a->blocks, kThreads, 0, stream>>>(*a);
             LF_CUDA(cudaGetLastError());
-            ic0_level_sweep<0><<<kSweepCluster, kSweepBlock, ap.smem, stream>>>(*a);
+            if (a->pipe_groups > 0) ic0_pipe_sweep<0><<<1, pipe_threads(*a), ap.smem, stream>>>(*a);
+            else ic0_level_sweep<0><<<kSweepCluster, kSweepBlock, ap.smem, stream>>>(*a);
         } else {
             ic0_forward<<<ap.chunks, kSweepRows, 0, stream>>>(*a);  // one CTA per chunk of kSweepRows rows
         }
         LF_CUDA(cudaGetLastError());
         trail.mark(in_loop ? 2 : -1);
-        if (ap.levels) {
+        if (ap.levels && a->pipe_groups > 0) {
+            ic0_pipe_sweep<1><<<1, pipe_threads(*a), ap.smem, stream>>>(*a);
+        } else if (ap.levels) {
             ic0_level_sweep<1><<<kSweepCluster, kSweepBlock, ap.smem, stream>>>(*a);
         } else {
             ic0_backward<<<ap.chunks, kSweepRows, 0, stream>>>(*a);
@@ -2261,6 +2536,16 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
     a.sw_maxe = c.sweep_maxe;
     SeparateApply ap{};
     ap.levels = true;
+    PipeShape pipe{};
+    const bool piped = ic0_use_pipe(c, fp32) && ic0_pipe_shape(c, fp32 ? 4 : 8, pipe);
+    if (piped) {
+        a.pipe_warps = pipe.group_warps;
+        a.pipe_groups = pipe.groups;
+        a.pipe_stages = pipe.stages;
+        a.sw_window = pipe.window;
+        a.sw_maxp = static_cast<int>(c.sweep_max_width);
+        a.sw_maxe = c.sweep_level_entries;
+    }
     if (fp32) {
         c.sweep_y32.ensure(c.n + kSweepSlack);
         c.sweep_rhs32.ensure(c.n + kSweepSlack);
@@ -2268,6 +2553,12 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         a.sw_y = c.sweep_y32.p;
         a.sw_rhs = c.sweep_rhs32.p;
         a.sw_rr = c.sweep_rr32.p;
+        if (piped) {
+            ap.smem = pipe.smem;
+            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            return ap;
+        }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(float)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
         LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
         LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
@@ -2276,6 +2567,12 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         c.sweep_rhs.ensure(c.n + kSweepSlack);
         a.sw_y = c.sweep_y.p;
         a.sw_rhs = c.sweep_rhs.p;
+        if (piped) {
+            ap.smem = pipe.smem;
+            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            return ap;
+        }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(double)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
         LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
         LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
@@ -2624,9 +2921,11 @@ void launch_precond_apply(Context& c, int precond, const double* r, double* z) {
         const SeparateApply ap = sweep_args(c, a, false);
         ic0_sweep_inputs<false><<<blocks, kThreads, 0, c.stream>>>(a);
         LF_CUDA(cudaGetLastError());
-        ic0_level_sweep<0><<<kSweepCluster, kSweepBlock, ap.smem, c.stream>>>(a);
+        if (a.pipe_groups > 0) ic0_pipe_sweep<0><<<1, pipe_threads(a), ap.smem, c.stream>>>(a);
+        else ic0_level_sweep<0><<<kSweepCluster, kSweepBlock, ap.smem, c.stream>>>(a);
         LF_CUDA(cudaGetLastError());
-        ic0_level_sweep<1><<<kSweepCluster, kSweepBlock, ap.smem, c.stream>>>(a);
+        if (a.pipe_groups > 0) ic0_pipe_sweep<1><<<1, pipe_threads(a), ap.smem, c.stream>>>(a);
+        else ic0_level_sweep<1><<<kSweepCluster, kSweepBlock, ap.smem, c.stream>>>(a);
         c.launches += 3;
     } else if (precond == LFGPU_PRECOND_IC0) {
         // The sweeps read the done flag of a solver state: give them a fresh one.

@@ -269,6 +269,7 @@ struct Context {
     int sweep_window = 0;             // ring slots (a power of two); 0: the schedule does not fit
     i64 sweep_max_width = 0, sweep_max_distance = 0;
     int sweep_maxp = 0, sweep_maxe = 0;  // the largest piece a CTA takes of a level: rows, entries
+    int sweep_level_entries = 0;         // entries of the level with the most
     Buf<double> sweep_y, sweep_rhs;   // forward result in backward positions; r in forward positions
     Buf<float> sweep_y32, sweep_rhs32, sweep_rr32;  // the same in FP32; r32 in backward positions
 

@@ -251,6 +251,7 @@ void ensure_ic0_schedule(Context& c) {
     c.sweep_max_distance = 0;
     c.sweep_maxp = 0;
     c.sweep_maxe = 0;
+    c.sweep_level_entries = 0;
     std::vector<int> pieces;
     for (int d = 0; d < 2; ++d) {
         const SweepSchedule& s = *both[d];
@@ -281,6 +282,8 @@ void ensure_ic0_schedule(Context& c) {
         for (int L = 0; L < s.levels; ++L) {
             const int p0 = s.level_begin[2 * static_cast<size_t>(L)], p1 = s.level_begin[2 * static_cast<size_t>(L) + 2];
             const int chunk = (p1 - p0 + kSweepCluster - 1) / kSweepCluster;
+            c.sweep_level_entries = std::max(c.sweep_level_entries, s.level_begin[2 * static_cast<size_t>(L) + 3] -
+                                                                        s.level_begin[2 * static_cast<size_t>(L) + 1]);
             for (int k = 0; k < kSweepCluster; ++k) {
                 const int first = std::min(p1, p0 + k * chunk), end = std::min(p1, first + chunk);
                 int* pc = &pieces[8 * (static_cast<size_t>(L) * kSweepCluster + k)];
@@ -344,16 +347,50 @@ void ensure_ic0_sweep_values(Context& c, bool fp32) {
     LF_CUDA(cudaGetLastError());
 }
 
-// LFGPU_IC0_SWEEP_AUTO takes the FP64 level sweeps where the forward schedule's
-// levels hold kLevelsMinWidth rows on average or more.  A level costs them about
-// 1.8 us whatever its width (one row's FP64 chain plus the exchange); the polled
-// sweeps' cost per level grows with it.  Per forward + backward application on
-// GB300 (cantilever workloads, RCM): 200x200, 50 rows a level: polled 3.9 ms,
-// levels 5.6 ms; 500x500, 125 rows: 13.3-13.6 ms, 14.1 ms; 1000x1000, 250 rows:
-// 30.5-30.9 ms, 28.4 ms.
+bool ic0_pipe_shape(const Context& c, int elem, PipeShape& s) {
+    const int width = static_cast<int>(c.sweep_max_width);
+    if (c.sweep_pattern_version != c.pattern_version || width < 1 || width > kPipeMaxWidth) return false;
+    s.group_warps = (width + 31) / 32;
+    s.groups = std::min(8, kPipeWarps / s.group_warps);
+    int optin = 0;
+    LF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c.device));
+    const int stage = sweep_stage_layout(elem, width, c.sweep_level_entries).bytes;
+    // A result is read up to max_distance positions on, while no warp is more than `stages`
+    // levels ahead of another.
+    for (s.stages = kPipeStages; s.stages >= s.groups + 2; --s.stages) {
+        const i64 need = c.sweep_max_distance + static_cast<i64>(s.stages + 2) * width;
+        s.window = 256;
+        while (s.window < need) s.window *= 2;
+        const i64 bytes = static_cast<i64>(s.window) * elem + static_cast<i64>(s.stages) * stage;
+        if (bytes <= optin - kSweepStaticSmem) {
+            s.smem = static_cast<int>(bytes);
+            return true;
+        }
+    }
+    return false;
+}
+
+bool ic0_use_pipe(const Context& c, bool fp32) {
+    PipeShape s;
+    return c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO &&
+           ic0_pipe_shape(c, fp32 ? static_cast<int>(sizeof(float)) : static_cast<int>(sizeof(double)), s);
+}
+
+// LFGPU_IC0_SWEEP_AUTO takes the pipelined sweeps where no level is wider than
+// kPipeMaxWidth rows and the schedule fits one CTA.  Per forward + backward application
+// on GB300 (cantilevers, RCM; polled / levels / pipelined): 96x96, up to 49 rows a level,
+// 1.77 / 2.74 / 0.62 ms; 250x250, 126 rows: 5.24 / 7.11 / 2.29; 500x500, 251 rows:
+// 13.95 / 14.34 / 7.61; a mixed iteration there, levels / pipelined: 1.07 / 0.40,
+// 2.75 / 1.39 and 5.58 / 5.03 ms, which is where the two meet.
+// Elsewhere FP64 takes the cluster's level sweeps where the forward schedule's levels
+// hold kLevelsMinWidth rows on average or more.  A level costs them about 1.8 us
+// whatever its width (one row's FP64 chain plus the exchange); the polled sweeps' cost
+// per level grows with it: at 500x500, 125 rows on average, polled 13.3-13.6 ms, levels
+// 14.1 ms; 1000x1000, 250 rows: 30.5-30.9 ms, 28.4 ms.
 constexpr i64 kLevelsMinWidth = 192;
 
 bool ic0_levels_chosen(const Context& c, bool required) {
+    if (c.sweep_pattern_version == c.pattern_version && ic0_use_pipe(c, required)) return true;
     if (c.sweep_window <= 0 || c.sweep_pattern_version != c.pattern_version) return false;
     if (required || c.ic0_sweep == LFGPU_IC0_SWEEP_LEVELS) return true;
     return c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO && c.n >= kLevelsMinWidth * c.sweep[0].levels;
@@ -364,7 +401,7 @@ bool ic0_use_levels(Context& c, bool required) {
     LF_REQUIRE(c.ic0_sweep != LFGPU_IC0_SWEEP_POLLED, LFGPU_ERR_UNSUPPORTED,
                "mixed-precision ic0 needs the level-scheduled sweeps");
     ensure_ic0_schedule(c);
-    if (c.sweep_window > 0) return ic0_levels_chosen(c, required);
+    if (c.sweep_window > 0 || ic0_use_pipe(c, required)) return ic0_levels_chosen(c, required);
     LF_REQUIRE(!required && c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO, LFGPU_ERR_UNSUPPORTED,
                "the ic0 level schedule does not fit the sweep's shared-memory ring");
     return false;

@@ -132,6 +132,22 @@ constexpr int kSweepStaticSmem = 4096;
 // rounded up to whole 16-byte units reads up to three elements beyond its range.
 constexpr int kSweepSlack = 16;
 
+// The pipelined level sweeps run in one CTA: groups of warps take the levels in turn,
+// a thread per row, and work on several levels at once.
+constexpr int kPipeWarps = 28;      // consumer warps at most
+constexpr int kPipeProducers = 4;   // warps that copy operands in
+constexpr int kPipeMaxWidth = 256;  // rows of the widest level they take
+constexpr int kPipeStages = 24;     // at most
+constexpr int kPipeDone = 64;       // mbarriers cycling over the levels' completions
+struct PipeShape {
+    int group_warps, groups, stages, window, smem;
+};
+// Their launch shape for elements of `elem` bytes; false when the schedule is too wide
+// or does not fit a CTA's shared memory.  Requires ensure_ic0_schedule.
+bool ic0_pipe_shape(const Context& c, int elem, PipeShape& s);
+// Whether they run (FP64: in place of the polled or the cluster's sweeps).
+bool ic0_use_pipe(const Context& c, bool fp32);
+
 // pattern.cu: CSR pattern and element->value map on the device; false if a node
 // has more elements than the device build handles (the caller builds on the host)
 bool build_pattern_device(Context& c, std::vector<int>& rowptr_host);
