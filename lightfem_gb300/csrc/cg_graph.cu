@@ -104,9 +104,11 @@ struct CgArgs {
     double* y;                     // IC(0) forward-sweep result
     unsigned long long* ic_chunks; // IC(0) row-chunk counters (forward, backward)
     const int* sub_dofs;           // subdomain block-Jacobi: DOFs by subdomain
+    const int* sub_order;          // the subdomains, largest first
     const int* sub_begin;
     const long long* sub_fac;      // packed lower factor offset of each subdomain
-    const double* sub_factor;
+    const double* sub_factor;      // by rows
+    const double* sub_factor_t;    // by columns
     const float* sub_inv32;        // mixed loop: block inverses, FP32 D x D squares
     const long long* sub_sq;       // offset of each subdomain's square
     // IC(0) level-scheduled sweeps (ic0.cu builds the schedules): [0] forward, [1] backward
@@ -1824,34 +1826,140 @@ __global__ void __launch_bounds__(kThreads) ic0_dot(CgArgs a) {
 }
 
 // One application z = M^-1 r of the subdomain block-Jacobi preconditioner
-// (SubdomainBlockJacobi::apply, src/precond.cpp:242-282): one CTA per subdomain,
-// thread i holding local row i.  Forward substitution with the packed lower
-// factor, then back substitution with its transpose, column by column: after
-// unknown j is final every later row subtracts its term, so each row subtracts
-// its terms in the reference's order (ascending forward, descending backward),
-// each product and difference rounded on its own.  The result equals the
-// reference's bit for bit.  The kernel is bound by the FP64 pipe: a separate
-// multiply and subtract per factor entry and sweep.
+// (SubdomainBlockJacobi::apply, src/precond.cpp:242-282): one CTA per subdomain, a
+// thread per local row.  Forward substitution with the packed lower factor, then back
+// substitution with its transpose, column by column: once unknown j is final every
+// later row subtracts its term, so each row subtracts its terms in the reference's
+// order (ascending forward, descending backward), each product and difference rounded
+// on its own.  The result equals the reference's bit for bit.
+//
+// An unknown is a chain of three FP64 instructions of 64 cycles (the pivot's product,
+// the next row's product and difference), and the FP64 pipe does one of them per 64
+// cycles on each quarter of the SM, whatever lanes are active, even none.  So a warp
+// subtracts the terms of the rows before its own 32 as they are published in shared
+// memory (a bounded poll of the value itself), then works its own unknowns out by
+// shuffles; no barrier holds the warp with the chain, and no warp issues terms it has
+// no rows for.  CTAs that share an SM start on different quarters, the largest
+// subdomains start first.  The factor's entries come a group or two ahead, a warp's 32
+// rows from consecutive addresses: forward from the copy by columns, backward from the
+// rows.  us an application, before (a barrier an unknown, predicated terms, both sweeps
+// along rows) and now, GB300, 64-node RCB blocks (up to 256 DOFs): 20x20, 7 blocks, 135
+// and 80 (the chain: 350 cycles an unknown); 180x160, 456 blocks, 300 and 102; 400x400,
+// 2513 blocks, 646 and 300 (the FP64 pipe), 1000x1000 5650 and 1711; 16-node blocks at 180x160 58 and 39.
+// Publishing a group at a time instead of each unknown: 84, 105 and 307.
+constexpr int kSubGroup = 4;
+// poll_shared where the value comes from another warp: no back-off.
+__device__ __forceinline__ double poll_warp(const volatile unsigned long long* p, DeviceStatus* status, int row) {
+    unsigned long long v = *p;
+    if (v == kPending) {
+        const unsigned long long t0 = global_ns();
+        for (unsigned it = 1; (v = *p) == kPending; ++it)
+            if ((it & 1023u) == 0u && wait_expired(status, t0, row)) break;
+    }
+    return __longlong_as_double(static_cast<long long>(v));
+}
 __global__ void __launch_bounds__(LFGPU_SUBDOMAIN_MAX_DOFS) subdomain_apply(CgArgs a) {
-    __shared__ double v[LFGPU_SUBDOMAIN_MAX_DOFS];
-    const int s = blockIdx.x, i = threadIdx.x;
+    __shared__ unsigned long long s_y[LFGPU_SUBDOMAIN_MAX_DOFS], s_z[LFGPU_SUBDOMAIN_MAX_DOFS];
+    const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int s = a.sub_order[blockIdx.x];
+    s_y[threadIdx.x] = s_z[threadIdx.x] = kPending;
+    __syncthreads();
+    // The warp's rows: rotated by the CTA's place in the grid.
+    const int turn = static_cast<int>(static_cast<long long>(blockIdx.x) * warps / gridDim.x);
+    const int first = 32 * ((threadIdx.x / 32 + turn) % warps), i = first + lane;
     const int begin = a.sub_begin[s], D = a.sub_begin[s + 1] - begin;
-    const double* __restrict__ f = a.sub_factor + a.sub_fac[s];
+    if (first >= D) return;
+    const double* __restrict__ by_row = a.sub_factor + a.sub_fac[s];
+    const double* __restrict__ by_col = a.sub_factor_t + a.sub_fac[s];
     const bool mine = i < D;
     const int dof = mine ? a.sub_dofs[begin + i] : 0;
-    const double* __restrict__ row = f + static_cast<long long>(i) * (i + 1) / 2;  // this thread's factor row
-    double acc = mine ? a.r[dof] : 0.0;
-    for (int j = 0; j < D; ++j) {
-        if (i == j) v[j] = __dmul_rn(acc, row[j]);  // row[j] is the reciprocal pivot
-        __syncthreads();
-        if (mine && i > j) acc = __dsub_rn(acc, __dmul_rn(row[j], v[j]));
+    const double inv = mine ? __ldg(by_row + i * (i + 1) / 2 + i) : 0.0;
+    // Unknowns come in pairs of groups: rows past D are rows of zeros.
+    const int end = (D + 2 * kSubGroup - 1) / (2 * kSubGroup) * (2 * kSubGroup), own = min(32, end - first);
+    double acc = mine ? a.r[dof] : 0.0, x = 0.0, c0[kSubGroup], c1[kSubGroup];
+
+    // Forward: entries (i, j) below the diagonal, j ascending.
+    int j = 0, at = i;
+    const int below = mine ? i : 0;
+    auto columns = [&](double* c) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u) {
+            c[u] = j < below ? __ldg(by_col + at) : 0.0;
+            at += D - 1 - j++;  // column j + 1 starts at its diagonal
+        }
+    };
+    auto subtract_y = [&](const double* c, int j0) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u)
+            acc = __dsub_rn(acc, __dmul_rn(c[u], poll_warp(s_y + j0 + u, a.status, i)));
+    };
+    // A row's own step ends its part: what the later steps do to its acc is not read.
+    auto solve_y = [&](const double* c, int l) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u) {
+            const double y = __dmul_rn(acc, inv);
+            acc = __dsub_rn(acc, __dmul_rn(c[u], __shfl_sync(0xffffffffu, y, l + u)));
+            if (lane == l + u) {
+                x = y;
+                reinterpret_cast<volatile unsigned long long*>(s_y)[i] = publishable(y);
+            }
+        }
+    };
+    columns(c0);
+    columns(c1);
+    for (int j0 = 0; j0 < first; j0 += 2 * kSubGroup) {
+        subtract_y(c0, j0);
+        columns(c0);
+        subtract_y(c1, j0 + kSubGroup);
+        columns(c1);
     }
-    acc = mine ? v[i] : 0.0;
-    double x = 0.0;
-    for (int k = D - 1; k >= 0; --k) {
-        if (i == k) v[k] = x = __dmul_rn(acc, row[k]);
-        __syncthreads();
-        if (i < k) acc = __dsub_rn(acc, __dmul_rn(f[static_cast<long long>(k) * (k + 1) / 2 + i], v[k]));
+    for (int l = 0; l < own; l += 2 * kSubGroup) {
+        solve_y(c0, l);
+        columns(c0);
+        solve_y(c1, l + kSubGroup);
+        columns(c1);
+    }
+
+    // Backward: entries (k, i) of the rows k > i, k descending.
+    acc = mine ? x : 0.0;
+    int k = end - 1;
+    at = k * (k + 1) / 2 + i;
+    auto rows = [&](double* c) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u) {
+            c[u] = k > i && k < D ? __ldg(by_row + at) : 0.0;
+            at -= k--;
+        }
+    };
+    auto subtract_z = [&](const double* c, int k0) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u)
+            acc = __dsub_rn(acc, __dmul_rn(c[u], poll_warp(s_z + k0 - u, a.status, i)));
+    };
+    auto solve_z = [&](const double* c, int l) {
+#pragma unroll
+        for (int u = 0; u < kSubGroup; ++u) {
+            const double z = __dmul_rn(acc, inv);
+            acc = __dsub_rn(acc, __dmul_rn(c[u], __shfl_sync(0xffffffffu, z, l - u)));
+            if (lane == l - u) {
+                x = z;
+                reinterpret_cast<volatile unsigned long long*>(s_z)[i] = publishable(z);
+            }
+        }
+    };
+    rows(c0);
+    rows(c1);
+    for (int k0 = end - 1; k0 >= first + 32; k0 -= 2 * kSubGroup) {
+        subtract_z(c0, k0);
+        rows(c0);
+        subtract_z(c1, k0 - kSubGroup);
+        rows(c1);
+    }
+    for (int l = own - 1; l >= 0; l -= 2 * kSubGroup) {
+        solve_z(c0, l);
+        rows(c0);
+        solve_z(c1, l - kSubGroup);
+        rows(c1);
     }
     if (mine) a.z[dof] = x;
 }
@@ -2505,9 +2613,11 @@ void launch_separate_unrolled(cudaStream_t stream, CgArgs* a, int blocks, const 
 // The subdomain arrays, and the apply kernel's launch shape.
 SeparateApply subdomain_args(Context& c, CgArgs& a) {
     a.sub_dofs = c.sub_dofs;
+    a.sub_order = c.sub_order;
     a.sub_begin = c.sub_begin;
     a.sub_fac = c.sub_fac_begin;
     a.sub_factor = c.sub_factor;
+    a.sub_factor_t = c.sub_factor_t;
     a.sub_inv32 = c.sub_inv32;
     a.sub_sq = c.sub_sq_begin;
     SeparateApply ap{};
