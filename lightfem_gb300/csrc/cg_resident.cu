@@ -97,7 +97,7 @@ struct ResArgs {
     int halo_cap;                // nodes of the arriving halo
     int own_cap;                 // nodes whose r and q are in shared memory (0: in global memory)
     int x_cap;                   // the same for the solution or its correction pair
-    int keep;                    // slices below this stay in L2, later ones stream
+    int keep;                    // of 16 slices this many stay in L2, the others stream
     u64* words;
     double* partials;
     u64* bar;
@@ -991,7 +991,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
         {
             Sum t[1] = {};
             each_node([&](int s, int node, int at) {
-                const V y = slice_row<CACHED>(a, s, node, win, node - w0, s < a.keep ? pol_keep : pol_stream);
+                const V y = slice_row<CACHED>(a, s, node, win, node - w0, (s & 15) < a.keep ? pol_keep : pol_stream);
                 const V p = own[at];
                 q[at] = y;
                 if constexpr (MIXED) t[0].add(p.x * y.x + p.y * y.y);
@@ -1447,6 +1447,22 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
     return true;
 }
 
+// Of 16 slices, how many are to stay in L2 between iterations: all while the matrix is
+// up to 4/5 of it, beyond that 3/10 of it, the rest of the L2 being the vectors' and the
+// stream's.  us an iteration on GB300 (129 MB of L2), all kept / 3/10 of L2 / none:
+// FP32 700x700 (83 MB) 14.1 / 18.9 / 20.3, 760x760 (97 MB) 19.3 / 19.8 / 21.4, 840x840
+// (119 MB) 32.4 / 24.4 / 25.4, 1000x1000 (169 MB) 44.1 / 34.4 / 34.9; FP64 560x560
+// (96 MB) 38.1 / 37.5 / 38.4, 640x640 (125 MB) 49.0 / 45.5 / 47.0.
+int keep_share(const Context& c, bool mixed) {
+    const size_t padded = static_cast<size_t>(slices_of(c)) * kSlice;
+    const size_t rows = static_cast<size_t>(c.resident.groups) * kSlice;
+    const double bytes = mixed ? 144.0 * rows + 24.0 * padded : 272.0 * rows + 32.0 * padded;
+    int l2 = 0;
+    LF_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
+    if (bytes <= 0.8 * l2) return 16;
+    return static_cast<int>(16.0 * 0.3 * l2 / bytes + 0.5);
+}
+
 bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms) {
     if (!c.paired || c.num_sms > 255 || c.n < 2) return false;
     const bool mixed = s.mixed != 0;
@@ -1514,7 +1530,7 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
     a.halo_cap = sh.halo_cap;
     a.own_cap = sh.own_cap;
     a.x_cap = sh.x_cap;
-    a.keep = slices;
+    a.keep = keep_share(c, mixed);
     if (sh.sync == kTagged) {
         const size_t words = padded * (mixed ? kTagWords<float2> : kTagWords<double2>);
         res.tagged.ensure(words);
