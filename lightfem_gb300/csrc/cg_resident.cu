@@ -44,9 +44,9 @@
 // cantilevers, log-normal moduli, RCM, Jacobi; GB300):
 //   n            8     20    50    80    100   200   300   400   500   640   800   1000
 //   FP64  graph  28.5        29.8        32.1  36.1  44.9  57.7        ~97         200
-//         here    4.8   4.9   5.6   6.0   7.2   8.5  14.2  22.0  29.8  48.7  74.3  106
+//         here    4.8   4.9   5.6   6.0   7.2   8.5  14.2  22.0  29.8  45.2  68.1  103
 //   mixed graph  20.9        20.0        20.1  21.5  24.2  24.5   28   ~33         58
-//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.6   7.4   8.3  11.3  34.1  49.3
+//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.6   7.4   8.3  11.3  21.8  33.7
 // FP64 is bound by the FP64 pipe from 200 on (52 instructions a node, 40 us at 640);
 // mixed by the crossings up to 400 and by HBM from 800 on, where K leaves L2.  With FP64
 // shuffles and FP64 scalars in the sums a mixed iteration took 3.9 us at 8, 6.0 at 50
@@ -878,6 +878,14 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
         reach_lo = s_reach[0];
         reach_hi = s_reach[1];
     }
+    // Of the CTA's matrix, what stays in L2 (keep_share).  FP32 waits for HBM and reads it
+    // last: interleaved 24.2 and 34.5 us an iteration at 840x840 and 1000x1000, last 23.0-24.3
+    // and 33.7 (by s mod 16 alone, always the same warps', 24.9 and 35.2).  FP64 shares its
+    // time with the pipe and has it interleaved: 45.2 us at 640x640, last 46.2.
+    auto keep_slice = [&](int s) {
+        if constexpr (MIXED) return (se - s) * 16 <= (se - sb) * a.keep;
+        else return ((s + 5 * (s >> 5)) & 15) < a.keep;
+    };
     // z of a node to whoever has it in a window; cluster: for the r.r and r.z sum in fixed
     // point (mbarrier 1) or in FP64 (3).
     int z_bar = 3;
@@ -991,7 +999,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
         {
             Sum t[1] = {};
             each_node([&](int s, int node, int at) {
-                const V y = slice_row<CACHED>(a, s, node, win, node - w0, (s & 15) < a.keep ? pol_keep : pol_stream);
+                const V y = slice_row<CACHED>(a, s, node, win, node - w0, keep_slice(s) ? pol_keep : pol_stream);
                 const V p = own[at];
                 q[at] = y;
                 if constexpr (MIXED) t[0].add(p.x * y.x + p.y * y.y);
@@ -1448,18 +1456,19 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
 }
 
 // Of 16 slices, how many are to stay in L2 between iterations: all while the matrix is
-// up to 4/5 of it, beyond that 3/10 of it, the rest of the L2 being the vectors' and the
-// stream's.  us an iteration on GB300 (129 MB of L2), all kept / 3/10 of L2 / none:
-// FP32 700x700 (83 MB) 14.1 / 18.9 / 20.3, 760x760 (97 MB) 19.3 / 19.8 / 21.4, 840x840
-// (119 MB) 32.4 / 24.4 / 25.4, 1000x1000 (169 MB) 44.1 / 34.4 / 34.9; FP64 560x560
-// (96 MB) 38.1 / 37.5 / 38.4, 640x640 (125 MB) 49.0 / 45.5 / 47.0.
+// up to 3/4 of it, beyond that 3/10 of it, the rest of the L2 being the vectors' and the
+// stream's.  us an iteration on GB300 (135 MB of L2), all kept / 3/10 of L2 / none:
+// FP32 700x700 (83 MB) 14.1 / 18.9 / 20.3, 760x760 (97 MB) 19.3 / 19.8 / 21.4, 800x800
+// (108 MB) 27.4 / 21.8 / -, 840x840 (119 MB) 32.4 / 24.3 / 25.4, 1000x1000 (169 MB)
+// 44.1 / 33.7 / 34.9; FP64 560x560
+// (96 MB) 38.1 / 37.5 / 38.4, 640x640 (125 MB) 49.0 / 45.4 / 47.0.
 int keep_share(const Context& c, bool mixed) {
     const size_t padded = static_cast<size_t>(slices_of(c)) * kSlice;
     const size_t rows = static_cast<size_t>(c.resident.groups) * kSlice;
     const double bytes = mixed ? 144.0 * rows + 24.0 * padded : 272.0 * rows + 32.0 * padded;
     int l2 = 0;
     LF_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
-    if (bytes <= 0.8 * l2) return 16;
+    if (bytes <= 0.75 * l2) return 16;
     return static_cast<int>(16.0 * 0.3 * l2 / bytes + 0.5);
 }
 
