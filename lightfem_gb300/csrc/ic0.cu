@@ -372,7 +372,7 @@ bool ic0_pipe_shape(const Context& c, int elem, PipeShape& s) {
 
 bool ic0_use_pipe(const Context& c, bool fp32) {
     PipeShape s;
-    return c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO &&
+    return c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO && c.sweep_window > 0 &&
            ic0_pipe_shape(c, fp32 ? static_cast<int>(sizeof(float)) : static_cast<int>(sizeof(double)), s);
 }
 
@@ -401,7 +401,7 @@ bool ic0_use_levels(Context& c, bool required) {
     LF_REQUIRE(c.ic0_sweep != LFGPU_IC0_SWEEP_POLLED, LFGPU_ERR_UNSUPPORTED,
                "mixed-precision ic0 needs the level-scheduled sweeps");
     ensure_ic0_schedule(c);
-    if (c.sweep_window > 0 || ic0_use_pipe(c, required)) return ic0_levels_chosen(c, required);
+    if (c.sweep_window > 0) return ic0_levels_chosen(c, required);
     LF_REQUIRE(!required && c.ic0_sweep == LFGPU_IC0_SWEEP_AUTO, LFGPU_ERR_UNSUPPORTED,
                "the ic0 level schedule does not fit the sweep's shared-memory ring");
     return false;
