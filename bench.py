@@ -618,7 +618,7 @@ def run_ours(args) -> int:
             ms, r = step(opts(prec, st, pc, pers))
             variants.append({"precision": prec, "storage": st, "preconditioner": pc,
                              **({"subdomain_nodes": 64, "subdomain_split": "rcb"} if pc == "subdomain" else {}),
-                             "loop": "persistent" if pers else "graph", "step_ms": round(ms, 2),
+                             "loop": "persistent" if pers else "resident", "step_ms": round(ms, 2),
                              "solve_ms": round(r.solve_ms, 2), "iterations": r.iterations,
                              "refinements": r.refinements, "true_residual_rel": r.true_residual / r.initial_residual,
                              "final_residual_rel": r.final_residual / r.initial_residual,
@@ -638,11 +638,10 @@ def run_ours(args) -> int:
             b = spmv_bytes(st + tag, n, nnz, nblocks)
             spmv[f"{st}{tag}"] = {"us": round(ms * 1e3, 2), "algorithmic_bytes": b, "gbs": round(b / ms / 1e6, 1)}
 
-    # Roofline of the dominant kernel of the step: the inner solve's FP32 product
-    # (mx_product, about half of the loop's device time).  The graph hides its
-    # launches from events, so the same loop runs once more with every kernel
-    # launched on the stream and an event after each launch; the product's average
-    # launch time comes from those events.
+    # Roofline of the FP32 product (mx_product).  The step's solve is one kernel, whose
+    # products no event can time; a profiling solve runs the same recurrence with every
+    # phase launched on the stream and an event after each launch, and the product's
+    # average launch time comes from those events.
     peaks = measured_peaks()
     ctx.assemble("coloring")
     ctx.apply_dirichlet()
@@ -707,7 +706,7 @@ def run_ours(args) -> int:
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+f64", "data": DATA,
             "config": {"workload": WORKLOAD, "precision": "mixed (FP32 inner PCG, FP64 refinement)",
                        "storage": args.storage, "preconditioner": args.precond, "tolerance": tol,
-                       "step": STEP_DESC, "loop": "device-driven CUDA graph (conditional WHILE)",
+                       "step": STEP_DESC, "loop": "one resident kernel per solve",
                        "l2": "inputs larger than L2 (K: 324 MB FP64 BSR, 162 MB FP32 BSR with 16-bit column offsets)"},
             "iterations": rep.iterations, "refinements": rep.refinements, "true_residual_rel": true_rel,
             "solve_ms": round(rep.solve_ms, 3),

@@ -110,7 +110,9 @@ typedef struct lfgpu_solve_options {
     int32_t refinement;        /* LFGPU_REFINE_* (mixed only) */
     double inner_reduction;    /* mixed: FP32 residual drop that triggers an FP64 update */
     int64_t max_refinements;   /* mixed: cap on FP64 residual replacements */
-    int32_t persistent;        /* 1: one persistent cooperative kernel; 0: device-driven CUDA graph of
+    int32_t persistent;        /* 1: the persistent kernel with TMA-staged products; 0: one resident kernel
+                                  for Jacobi and 2x2 blocks, where the pattern is paired and its rows'
+                                  columns fit a window in shared memory, else a device-driven CUDA graph of
                                   per-phase kernels (conditional WHILE node) */
     int32_t unrolled;          /* profiling only, graph loop: > 0 replaces the conditional loop by a plain
                                   graph of this many iterations (profilers do not descend into
