@@ -44,9 +44,9 @@
 // cantilevers, log-normal moduli, RCM, Jacobi; GB300):
 //   n            8     20    50    80    100   200   300   400   500   640   800   1000
 //   FP64  graph  28.5        29.8        32.1  36.1  44.9  57.7        ~97         200
-//         here    4.8   4.9   5.6   6.0   7.2   8.5  14.2  22.0  29.8  45.2  68.1  103
+//         here    4.8   4.9   5.6   6.0   7.2   8.5  13.7  20.3  29.4  45.2  68.1  103
 //   mixed graph  20.9        20.0        20.1  21.5  24.2  24.5   28   ~33         58
-//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.6   7.4   8.3  11.3  21.8  33.7
+//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.1   7.1   7.9  11.3  21.8  33.7
 // FP64 is bound by the FP64 pipe from 200 on (52 instructions a node, 40 us at 640);
 // mixed by the crossings up to 400 and by HBM from 800 on, where K leaves L2.  With FP64
 // shuffles and FP64 scalars in the sums a mixed iteration took 3.9 us at 8, 6.0 at 50
@@ -1382,6 +1382,23 @@ Shape launch_shape(const Context& c, bool mixed) {
 
 }  // namespace
 
+// Of 16 slices, how many are to stay in L2 between iterations: all while the matrix is
+// up to 3/4 of it, beyond that 3/10 of it, the rest of the L2 being the vectors' and the
+// stream's.  us an iteration on GB300 (135 MB of L2), all kept / 3/10 of L2 / none:
+// FP32 700x700 (83 MB) 14.1 / 18.9 / 20.3, 760x760 (97 MB) 19.3 / 19.8 / 21.4, 800x800
+// (108 MB) 27.4 / 21.8 / -, 840x840 (119 MB) 32.4 / 24.3 / 25.4, 1000x1000 (169 MB)
+// 44.1 / 33.7 / 34.9; FP64 560x560
+// (96 MB) 38.1 / 37.5 / 38.4, 640x640 (125 MB) 49.0 / 45.4 / 47.0.
+int keep_share(const Context& c, bool mixed) {
+    const size_t padded = static_cast<size_t>(slices_of(c)) * kSlice;
+    const size_t rows = static_cast<size_t>(c.resident.groups) * kSlice;
+    const double bytes = mixed ? 144.0 * rows + 24.0 * padded : 272.0 * rows + 32.0 * padded;
+    int l2 = 0;
+    LF_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
+    if (bytes <= 0.75 * l2) return 16;
+    return static_cast<int>(16.0 * 0.3 * l2 / bytes + 0.5);
+}
+
 // The slices and windows of the current pattern; false when the resident kernel does
 // not take it.
 static bool resident_structure(Context& c, bool mixed, Shape& s) {
@@ -1423,8 +1440,6 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
     // The CTA's matrix share fits L1 beside its shared memory.
     const int row_bytes = mixed ? 8 * 16 + 16 + 16 + 8 + 12 : 8 * 32 + 32 + 16 + 24;
     s.cached = s.sync == kCluster || own * row_bytes + s.smem < optin - 24 * 1024;
-    s.threads = 32 * std::max(s.sync == kCluster ? 1 : 4,
-                              std::min(max_threads(mixed, s.cached) / 32, own / kSlice));
     if (res.pattern_version != c.pattern_version) {
         int groups = slices;
         res.uniform = grid.info[1] <= kGroup + 1;
@@ -1452,24 +1467,18 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
         res.pattern_version = c.pattern_version;
         res.k_version[0] = res.k_version[1] = ~0ull;
     }
+    // Warps take the CTA's slices in rounds: no more warps than the rounds can use evenly,
+    // in pairs (400x400, 33 slices: 18 warps twice rather than 32 and one).  us an iteration
+    // on GB300 with as many as fit and so: mixed 300x300 5.8, 5.1; 400x400 7.9, 7.1; 560x560
+    // 10.1, 9.05; FP64 300x300 14.4, 13.6; 400x400 21.9, 20.3; 560x560 38.2, 36.9.  A mixed
+    // solve that waits for HBM wants the loads of all: 840x840 24.1, 24.7; 1000x1000 33.8, 34.9.
+    int warps = std::min(max_threads(mixed, s.cached) / 32, own / kSlice);
+    if (!(mixed && keep_share(c, mixed) < 16)) {
+        const int rounds = (own / kSlice + warps - 1) / warps;
+        warps = std::min(warps, ((own / kSlice + rounds - 1) / rounds + 1) & ~1);
+    }
+    s.threads = 32 * std::max(s.sync == kCluster ? 1 : 4, warps);
     return true;
-}
-
-// Of 16 slices, how many are to stay in L2 between iterations: all while the matrix is
-// up to 3/4 of it, beyond that 3/10 of it, the rest of the L2 being the vectors' and the
-// stream's.  us an iteration on GB300 (135 MB of L2), all kept / 3/10 of L2 / none:
-// FP32 700x700 (83 MB) 14.1 / 18.9 / 20.3, 760x760 (97 MB) 19.3 / 19.8 / 21.4, 800x800
-// (108 MB) 27.4 / 21.8 / -, 840x840 (119 MB) 32.4 / 24.3 / 25.4, 1000x1000 (169 MB)
-// 44.1 / 33.7 / 34.9; FP64 560x560
-// (96 MB) 38.1 / 37.5 / 38.4, 640x640 (125 MB) 49.0 / 45.4 / 47.0.
-int keep_share(const Context& c, bool mixed) {
-    const size_t padded = static_cast<size_t>(slices_of(c)) * kSlice;
-    const size_t rows = static_cast<size_t>(c.resident.groups) * kSlice;
-    const double bytes = mixed ? 144.0 * rows + 24.0 * padded : 272.0 * rows + 32.0 * padded;
-    int l2 = 0;
-    LF_CUDA(cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, c.device));
-    if (bytes <= 0.75 * l2) return 16;
-    return static_cast<int>(16.0 * 0.3 * l2 / bytes + 0.5);
 }
 
 bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms) {
