@@ -515,8 +515,9 @@ struct GridSync {
 
 // The sum over all CTAs of K per-thread values of quantities FIRST.., then
 // fin(totals) on thread 0 of every CTA; false when a wait ran out.  FAST: in fixed
-// point at the scales of the last totals, where they allow it.  PUBLISH (grid): the
-// CTAs' earlier global writes are visible to all after it.  halo_bytes (cluster): z
+// point at the scales of the last totals, where they allow it.  PUBLISH: on the grid the
+// CTAs' earlier global writes are visible to all after it; in a cluster only what the
+// peers sent here is (meet() orders global memory there).  halo_bytes (cluster): z
 // that the peers send for this sum.  it: the iteration, for the words' set.
 // meanwhile(): work of the warps past the first while warp 0 waits.  Consecutive sums
 // use different slots: a peer that is one sum ahead then cannot reach this one's.
@@ -636,6 +637,20 @@ __device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync
         }
     }
     return sh.state != 0 && sh.fail == 0;
+}
+
+// All CTAs' earlier global writes are visible to all after it (reads past L1); false when
+// a wait ran out.  Through the counter in L2 in a cluster too: what its sums send to an
+// mbarrier orders the peers' shared memory and nothing else.
+__device__ __forceinline__ bool meet(const ResArgs& a, ResShared& sh, GridSync& g) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double none[1] = {0.0};
+        const bool ok = a.grid == 1 || g.plain<1>(none);
+        if (threadIdx.x == 0) sh.state = ok;
+    }
+    __syncthreads();
+    return sh.state != 0;
 }
 
 // ------------------------------------------------------------------ rows
@@ -1111,9 +1126,8 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
                 xs[at] = V{};
                 xl[at] = V{};
             });
-            double none[1] = {0.0};
-            if (!reduce<SYNC, false, kPq, 1, true, false>(a, sh, g, s_red, none, 0u, 0u, nothing, [](const double*) {}))
-                return false;
+            // The residual reads x of the other CTAs' nodes.
+            if (!meet(a, sh, g)) return false;
             double t[2] = {0.0, 0.0};
             tag += 1;
             z_bar = 3;
