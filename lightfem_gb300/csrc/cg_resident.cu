@@ -476,21 +476,30 @@ struct GridSync {
         return true;
     }
 
-    // A lane's word added over the CTAs (live lanes: 2 k and 2 k + 1).
-    // Words: the set's, and the ones CTA 0 clears for two iterations on.  Their last
-    // readers are past them, and CTA 0 sees the old values before it arrives at
-    // another sum, so nobody adds to a word before it is cleared.
-    template <bool PUBLISH>
-    __device__ __forceinline__ bool packed(u64& word, bool live, u64* set, u64* clear) {
+    // CTA 0, warp 0: clears the words of the sets two iterations on, in every iteration and
+    // whichever way its r.r and r.z sum is formed.  Their last readers are past them, and CTA
+    // 0 sees the old values (answered()) before it arrives at another sum, so nobody adds to
+    // a word before it is cleared.
+    __device__ __forceinline__ u64 clear_ahead(unsigned it) {
         const int lane = threadIdx.x & 31;
         u64 old = 0;
-        int ok = 1;
-        const u64 n = static_cast<u64>(grid);
-        if (clear != nullptr && blockIdx.x == 0 && lane >= 8 && lane < 14) {
+        if (blockIdx.x == 0 && lane >= 8 && lane < 14) {
             // Two words of a p.q set, four of an r.r and r.z set.
-            u64* w = lane < 10 ? clear + (lane - 8) : clear + kSets * kSetStride + (lane - 10);
+            u64* w = words + ((it + 2) & (kSets - 1)) * kSetStride +
+                     (lane < 10 ? lane - 8 : kSets * kSetStride + lane - 10);
             asm volatile("atom.relaxed.gpu.global.exch.b64 %0, [%1], %2;" : "=l"(old) : "l"(w), "l"(0ull) : "memory");
         }
+        return old;
+    }
+    // Waits for the exchange's answer; always true: no word counts 255 arrivals.
+    static __device__ __forceinline__ bool answered(u64 old) { return (old >> 56) != 255ull; }
+
+    // A lane's word added over the CTAs (live lanes: 2 k and 2 k + 1).
+    template <bool PUBLISH>
+    __device__ __forceinline__ bool packed(u64& word, bool live, u64* set) {
+        const int lane = threadIdx.x & 31;
+        int ok = 1;
+        const u64 n = static_cast<u64>(grid);
         if (live) {
             red_add<PUBLISH>(set + lane, word);
             ok = spin(status, limit, [&] {
@@ -498,7 +507,6 @@ struct GridSync {
                 return (word >> 56) == n;
             });
         }
-        ok = ok && (old >> 56) != 255ull;  // never 255: waits for the exchange's answer
         return __all_sync(0xffffffffu, ok) != 0;
     }
 
@@ -572,8 +580,9 @@ __device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync
                 }
             } else {
                 u64* set = a.words + ((FIRST == kPq ? 0 : kSets) + (it & (kSets - 1))) * kSetStride;
-                u64* clear = FIRST == kPq ? nullptr : a.words + ((it + 2) & (kSets - 1)) * kSetStride;
-                ok = g.packed<PUBLISH>(word, live, set, clear);
+                const u64 old = FIRST == kRr ? g.clear_ahead(it) : 0ull;
+                ok = g.packed<PUBLISH>(word, live, set);
+                ok = __all_sync(0xffffffffu, ok && GridSync::answered(old)) != 0;
             }
             Total<MIXED> mt;
             bool good = from_words(sh, FIRST + k, word, a.grid, mt);
@@ -618,7 +627,10 @@ __device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync
                 for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < a.grid ? sh.xch[kSlot][k][lane] : 0.0);
             }
         } else {
-            ok = g.plain<K>(v);
+            if constexpr (FAST && FIRST == kRr) {
+                if (!fast) ok = __all_sync(0xffffffffu, GridSync::answered(g.clear_ahead(it))) != 0;  // not yet done above
+            }
+            ok = g.plain<K>(v) && ok;
         }
         if (lane == 0) {
             if (ok) {
