@@ -2279,7 +2279,7 @@ StagedShape staged_shape(int nb) {
     const int grid = kStagedCtasPerSm * sms;
     const int stash = std::max(0, std::min((share - stages) / 16, staged_per_cta(nb, grid)));
     StagedShape sh{grid, stages + 16 * stash, stash};
-    LF_CUDA(cudaFuncSetAttribute(mx_update_staged<PRECOND>, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem));
+    allow_dynamic_smem(mx_update_staged<PRECOND>);
     LF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_update_staged<PRECOND>, kStagedBlock, sh.smem));
     LF_REQUIRE(per_sm >= 1, LFGPU_ERR_CUDA, "the staged update does not fit an SM");
     sh.grid = std::min(grid, per_sm * sms);
@@ -2665,13 +2665,13 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         a.sw_rr = c.sweep_rr32.p;
         if (piped) {
             ap.smem = pipe.smem;
-            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
-            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            allow_dynamic_smem(ic0_pipe_sweep<2>);
+            allow_dynamic_smem(ic0_pipe_sweep<3>);
             return ap;
         }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(float)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
-        LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
-        LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+        allow_dynamic_smem(ic0_level_sweep<2>);
+        allow_dynamic_smem(ic0_level_sweep<3>);
     } else {
         c.sweep_y.ensure(c.n + kSweepSlack);
         c.sweep_rhs.ensure(c.n + kSweepSlack);
@@ -2679,13 +2679,13 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         a.sw_rhs = c.sweep_rhs.p;
         if (piped) {
             ap.smem = pipe.smem;
-            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
-            LF_CUDA(cudaFuncSetAttribute(ic0_pipe_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+            allow_dynamic_smem(ic0_pipe_sweep<0>);
+            allow_dynamic_smem(ic0_pipe_sweep<1>);
             return ap;
         }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(double)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
-        LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
-        LF_CUDA(cudaFuncSetAttribute(ic0_level_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ap.smem));
+        allow_dynamic_smem(ic0_level_sweep<0>);
+        allow_dynamic_smem(ic0_level_sweep<1>);
     }
     return ap;
 }

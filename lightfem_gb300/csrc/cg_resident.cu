@@ -1605,9 +1605,7 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
     a.max_ref = s.max_refinements;
     a.restart = s.restart;
     auto launch = [&](auto kernel) {
-        LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sh.smem));
-        LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     std::min(100, (sh.smem + kStaticSmem32) * 100 / (228 * 1024) + 1)));
+        allow_dynamic_smem(kernel);
         if (sh.sync == kCluster && sh.grid > 8)
             LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};
@@ -1615,7 +1613,9 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
         cfg.blockDim = dim3(sh.threads);
         cfg.dynamicSmemBytes = sh.smem;
         cfg.stream = c.stream;
-        cudaLaunchAttribute attr[1] = {};
+        cudaLaunchAttribute attr[2] = {};
+        attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;  // the rest of the SM's memory is L1
+        attr[1].val.sharedMemCarveout = std::min(100, (sh.smem + kStaticSmem32) * 100 / (228 * 1024) + 1);
         if (sh.sync == kCluster) {
             attr[0].id = cudaLaunchAttributeClusterDimension;
             attr[0].val.clusterDim.x = sh.grid;
@@ -1625,7 +1625,7 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
             attr[0].val.cooperative = 1;
         }
         cfg.attrs = attr;
-        cfg.numAttrs = 1;
+        cfg.numAttrs = 2;
         LF_CUDA(cudaEventRecord(c.ev_a, c.stream));
         LF_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
         LF_CUDA(cudaEventRecord(c.ev_b, c.stream));
