@@ -491,8 +491,12 @@ struct GridSync {
         }
         return old;
     }
-    // Waits for the exchange's answer; always true: no word counts 255 arrivals.
-    static __device__ __forceinline__ bool answered(u64 old) { return (old >> 56) != 255ull; }
+    // Waits for the exchange's answer, here and not before (CTA 0 would hold up the others);
+    // always true: no word counts 255 arrivals.
+    static __device__ __forceinline__ bool answered(u64 old) {
+        asm volatile("" : "+l"(old)::"memory");
+        return (old >> 56) != 255ull;
+    }
 
     // A lane's word added over the CTAs (live lanes: 2 k and 2 k + 1).
     template <bool PUBLISH>
@@ -657,9 +661,12 @@ __device__ __forceinline__ bool reduce(const ResArgs& a, ResShared& sh, GridSync
 __device__ __forceinline__ bool meet(const ResArgs& a, ResShared& sh, GridSync& g) {
     __syncthreads();
     if (threadIdx.x < 32) {
-        double none[1] = {0.0};
-        const bool ok = a.grid == 1 || g.plain<1>(none);
-        if (threadIdx.x == 0) sh.state = ok;
+        g.arrivals += a.grid;
+        if (threadIdx.x == 0) {
+            red_add<true>(a.bar, 1ull);
+            const u64 want = g.arrivals;
+            sh.state = spin(a.status, g.limit, [&] { return ld_acquire(a.bar) >= want; });
+        }
     }
     __syncthreads();
     return sh.state != 0;
