@@ -51,6 +51,7 @@
 // mixed by the crossings up to 400 and by HBM from 800 on, where K leaves L2.  With FP64
 // shuffles and FP64 scalars in the sums a mixed iteration took 3.9 us at 8, 6.0 at 50
 // and 7.6 at 200, an FP64 one 6.3, 7.8 and 11.2.
+#include "cg_fixed.hpp"
 #include "cg_math.cuh"
 #include "common.cuh"
 #include "kernels.hpp"
@@ -192,24 +193,6 @@ __device__ __forceinline__ void quotient(PairTotal num, PairTotal den, float& hi
     lo = __fsub_rn(q2, __fsub_rn(hi, q1));
 }
 
-// Fixed point.  A share of a sum is cut into limbs of 21 bits (FP32 pairs: three, in
-// units of 2^-15, 2^-36 and 2^-56 of the scale 2^e) or 22 bits (FP64: four, in units
-// of 2^-70, 2^-48, 2^-26 and 2^-4), each a 32-bit integer that a warp adds with one
-// instruction; 1024 threads' limbs do not overflow.
-template <bool MIXED>
-constexpr int kLimbs = MIXED ? 3 : 4;
-constexpr int kScaleBits = 70;   // FP64: bits below the scale
-constexpr int kNoScale = 1 << 20;
-// Exponent of a positive normal total with room for the arithmetic around it, or kNoScale.
-__device__ __forceinline__ int exponent_of(double v) {
-    const int e = static_cast<int>(static_cast<u64>(bits_of(v)) >> 52);  // the sign counts too
-    return e > 123 && e < 1923 ? e - 1023 : kNoScale;
-}
-__device__ __forceinline__ int exponent_of(PairTotal v) {
-    const int e = static_cast<int>(__float_as_uint(v.hi) >> 23);
-    return e > 0 && e < 250 ? e - 127 : kNoScale;
-}
-
 struct ResShared {
     int e[3];                    // scales of the sums: exponents of the last totals (p.q, r.r, r.z)
     float up[3], down[3][2];     // mixed: 2^-e, and 2^(e - 36) as a product of two floats
@@ -229,14 +212,9 @@ struct ResShared {
 
 __device__ __forceinline__ void set_scale(ResShared& sh, int k, double t) { sh.e[k] = exponent_of(t); }
 __device__ __forceinline__ void set_scale(ResShared& sh, int k, PairTotal t) {
-    const int e = exponent_of(t);
+    const int e = exponent_of_pair(t.hi);
     sh.e[k] = e;
-    if (e != kNoScale) {  // e in [-126, 122]
-        sh.up[k] = __int_as_float((127 - e) << 23);
-        const int n = e - 36, a = n >> 1;
-        sh.down[k][0] = __int_as_float((a + 127) << 23);
-        sh.down[k][1] = __int_as_float((n - a + 127) << 23);
-    }
+    if (e != kNoScale) pair_scale(e, sh.up[k], sh.down[k]);
 }
 
 __device__ __forceinline__ u64 ld_relaxed(const u64* p) {
@@ -272,105 +250,23 @@ __device__ __forceinline__ bool spin(DeviceStatus* status, u64 limit, Read&& rea
     }
 }
 
-// The limbs of a thread's share; false when it is out of range.  FP32 pair: each limb
-// is the remainder so far rounded to the limb's unit, by adding 1.5 x 2^23, and the
-// remainders are exact.  |share| < 2^5 of the scale.
+// A thread's share in limbs, and a total from the words' sums over n CTAs (low in even
+// lanes, high in odd ones), in both lanes; false out of range (cg_fixed.hpp).
 __device__ __forceinline__ bool to_limbs(const ResShared& sh, int k, const FloatPair& v, int (&l)[3]) {
-    constexpr float kRound = 12582912.f;
-    constexpr int kBits = 0x4b400000;
-    const float hi = __fmul_rn(v.hi, sh.up[k]), lo = __fmul_rn(v.lo, sh.up[k]);
-    const float a = __fmaf_rn(hi, 0x1p15f, kRound);
-    const float r = __fmaf_rn(__fsub_rn(a, kRound), -0x1p-15f, hi);
-    const float b = __fmaf_rn(r, 0x1p36f, kRound), c = __fmaf_rn(lo, 0x1p36f, kRound);
-    const float s = __fmaf_rn(__fsub_rn(b, kRound), -0x1p-36f, r), t = __fmaf_rn(__fsub_rn(c, kRound), -0x1p-36f, lo);
-    l[2] = __float_as_int(a) - kBits;
-    l[1] = (__float_as_int(b) - kBits) + (__float_as_int(c) - kBits);
-    l[0] = __float_as_int(__fmaf_rn(__fadd_rn(s, t), 0x1p56f, kRound)) - kBits;
-    return fabsf(hi) < 0x1p5f && fabsf(lo) < 0x1p-17f;
+    return pair_limbs(sh.up[k], v.hi, v.lo, l);
 }
-// FP64: the mantissa shifted to its place in units of 2^-70 of the scale.  |share| <
-// 2^17 of the scale.
 __device__ __forceinline__ bool to_limbs(const ResShared& sh, int k, double v, int (&l)[4]) {
-    const u64 b = static_cast<u64>(bits_of(v));
-    const int ex = static_cast<int>((b >> 52) & 0x7ff);
-    const u64 m = (b & 0xfffffffffffffull) | (ex ? 1ull << 52 : 0ull);
-    const int n = max(ex, 1) - 1075 + kScaleBits - sh.e[k];
-    const bool ok = ex != 0x7ff && (m == 0 || n <= 34);
-    const int up = min(max(n, 0), 34), dn = min(max(-n, 0), 63);
-    const u64 lo = dn > 0 ? (m + (1ull << (dn - 1))) >> dn : m << up;
-    const u64 hi = up > 0 ? m >> (64 - up) : 0ull;
-    constexpr unsigned mask = 0x3fffffu;
-    const int l0 = static_cast<int>(static_cast<unsigned>(lo) & mask);
-    const int l1 = static_cast<int>(static_cast<unsigned>(lo >> 22) & mask);
-    const int l2 = static_cast<int>((static_cast<unsigned>(lo >> 44) | (static_cast<unsigned>(hi) << 20)) & mask);
-    const int l3 = static_cast<int>(hi >> 2);
-    const int sign = static_cast<int>(static_cast<long long>(b) >> 63);  // 0 or -1
-    l[0] = (l0 ^ sign) - sign;
-    l[1] = (l1 ^ sign) - sign;
-    l[2] = (l2 ^ sign) - sign;
-    l[3] = (l3 ^ sign) - sign;
-    return ok;
-}
-
-// A CTA's sum of a quantity travels in two words, low and high (a sector holds the four
-// words of r.r and r.z): arrivals in the top byte, CTAs out of range in the next, and
-// below them 40 bits of the sum, or the rest plus 2^39; 48 bits hold 255 CTAs' shares.
-// Units: 2^-56 of the scale (pairs), 2^-62 (FP64, rounded from the threads' 2^-70).
-constexpr long long kHighBias = 1ll << 39;
-constexpr long long kLowMask = (1ll << 40) - 1;
-template <bool MIXED>
-__device__ __forceinline__ u64 sum_word(const int* l, bool high, bool bad) {
-    long long lo, hi;
-    if (MIXED) {
-        lo = static_cast<long long>(l[0]) + (static_cast<long long>(l[1]) << 20) + (static_cast<long long>(l[2]) << 41);
-        hi = 0;
-    } else {
-        hi = static_cast<long long>(l[2]) + (static_cast<long long>(l[3]) << 22);  // units of 2^44
-        lo = (static_cast<long long>(l[0]) + (static_cast<long long>(l[1]) << 22) + 128) >> 8;
-        lo += (hi & 15) << 36;
-        hi >>= 4;
-    }
-    hi += lo >> 40;
-    lo &= kLowMask;
-    bad = bad || hi >= kHighBias || hi < -kHighBias;
-    return (1ull << 56) | (bad ? 1ull << 48 : 0ull) | (high ? (bad ? 0ull : static_cast<u64>(hi + kHighBias)) : static_cast<u64>(lo));
-}
-
-// A quantity's total from its two words' sums over n CTAs (low in even lanes, high in
-// odd ones), in both lanes; false when it is not positive and within ten bits of the
-// scale (then it is formed in FP64).
-__device__ __forceinline__ void halves(u64 word, int n, long long& lo, long long& hi) {
-    const u64 other = __shfl_xor_sync(0xffffffffu, word, 1);
-    const bool odd = threadIdx.x & 1;
-    lo = static_cast<long long>((odd ? other : word) & 0xffffffffffffull);
-    hi = static_cast<long long>((odd ? word : other) & 0xffffffffffffull) - n * kHighBias;
+    return fp64_limbs(sh.e[k], v, l);
 }
 __device__ __forceinline__ bool from_words(const ResShared& sh, int k, u64 word, int n, PairTotal& out) {
-    long long lo, hi;
-    halves(word, n, lo, hi);
-    const bool ok = hi > -(1ll << 20) && hi < (1ll << 20);
-    const long long s = (hi << 40) + lo;  // units of 2^-56
-    // Parts of 20 or 21 bits, exact in FP32; their sum as a pair in units of 2^-36.
-    const float f2 = static_cast<float>(static_cast<int>(s >> 41));
-    const float f1 = static_cast<float>(static_cast<int>(s >> 20) & 0x1fffff);
-    const float f0 = static_cast<float>(static_cast<int>(s) & 0xfffff);
-    const float h = __fmaf_rn(f2, 0x1p21f, f1);
-    const float l = __fmaf_rn(f0, 0x1p-20f, __fadd_rn(__fmaf_rn(f2, 0x1p21f, -h), f1));
-    out.hi = __fmul_rn(__fmul_rn(h, sh.down[k][0]), sh.down[k][1]);
-    out.lo = __fmul_rn(__fmul_rn(l, sh.down[k][0]), sh.down[k][1]);
-    return ok && s >= (1ll << 46);
+    const u64 other = __shfl_xor_sync(0xffffffffu, word, 1);
+    const bool odd = threadIdx.x & 1;
+    return pair_total(sh.down[k], odd ? other : word, odd ? word : other, n, out.hi, out.lo);
 }
 __device__ __forceinline__ bool from_words(const ResShared& sh, int k, u64 word, int n, double& out) {
-    long long lo, hi;
-    halves(word, n, lo, hi);
-    hi += lo >> 40;
-    lo &= kLowMask;
-    const bool ok = hi >= (1ll << 12) && hi < (1ll << 45);
-    const int lead = __clzll(hi);  // 19 to 51
-    const u64 w = (static_cast<u64>(hi) << lead) | ((static_cast<u64>(lo) << 24) >> ((64 - lead) & 63));
-    const u64 m = (w >> 11) + ((w >> 10) & 1);  // 53 bits, rounded
-    out = __longlong_as_double((static_cast<long long>(1023 + 41 - lead + sh.e[k] - 1) << 52) + static_cast<long long>(m));
-    return ok;
+    const u64 other = __shfl_xor_sync(0xffffffffu, word, 1);
+    const bool odd = threadIdx.x & 1;
+    return fp64_total(sh.e[k], odd ? other : word, odd ? word : other, n, out);
 }
 
 // Per-thread values to the CTA's totals in FP64, in all lanes of warp 0.
@@ -825,6 +721,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
     using Sum = typename std::conditional<MIXED, FloatPair, double>::type;
     using Tot = Total<MIXED>;
     constexpr bool kPublish = SYNC == kPublished;
+    static_assert(max_threads(MIXED, CACHED) <= kLimbThreads<MIXED>, "the CTA's limb sums would overflow");
     extern __shared__ __align__(16) unsigned char res_smem[];
     __shared__ ResShared sh;
     __shared__ double s_red[2 * max_threads(MIXED, CACHED)];
