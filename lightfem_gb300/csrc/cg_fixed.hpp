@@ -44,14 +44,14 @@ LF_FIXED int fx_clz(long long v) { return v == 0 ? 64 : __builtin_clzll(static_c
 
 // A share of a sum is cut into limbs of 21 bits (FP32 pairs: three, in
 // units of 2^-15, 2^-36 and 2^-56 of the scale 2^e) or 22 bits (FP64: four, in units
-// of 2^-70, 2^-48, 2^-26 and 2^-4), each a 32-bit integer that a warp adds with one
+// of 2^-78, 2^-56, 2^-34 and 2^-12), each a 32-bit integer that a warp adds with one
 // instruction: no more than 1024 threads (FP32 pairs) or 512 (FP64), then no sum of limbs
 // overflows.
 template <bool MIXED>
 constexpr int kLimbs = MIXED ? 3 : 4;
 template <bool MIXED>
 constexpr int kLimbThreads = MIXED ? 1024 : 512;
-constexpr int kScaleBits = 70;   // FP64: bits below the scale
+constexpr int kScaleBits = 78;   // FP64: bits below the scale
 constexpr int kNoScale = 1 << 20;
 
 // Exponent of a positive normal total with room for the arithmetic around it, or kNoScale.
@@ -87,8 +87,8 @@ LF_FIXED bool pair_limbs(float up, float vhi, float vlo, int (&l)[3]) {
     l[0] = fx_bits(fx_fma(fx_add(s, t), 0x1p56f, kRound)) - kBits;
     return fabsf(hi) < 0x1p5f && fabsf(lo) < 0x1p-17f;
 }
-// FP64: the mantissa shifted to its place in units of 2^-70 of the scale.  |share| <
-// 2^17 of the scale.
+// FP64: the mantissa shifted to its place in units of 2^-78 of the scale.  |share| <
+// 2^9 of the scale.
 LF_FIXED bool fp64_limbs(int e, double v, int (&l)[4]) {
     const unsigned long long b = static_cast<unsigned long long>(fx_bits(v));
     const int ex = static_cast<int>((b >> 52) & 0x7ff);
@@ -114,7 +114,9 @@ LF_FIXED bool fp64_limbs(int e, double v, int (&l)[4]) {
 // A CTA's sum of a quantity travels in two words, low and high (a sector holds the four
 // words of r.r and r.z): arrivals in the top byte, CTAs out of range in the next, and
 // below them 40 bits of the sum, or the rest plus 2^39; 48 bits hold 255 CTAs' shares.
-// Units: 2^-56 of the scale (pairs), 2^-62 (FP64, rounded from the threads' 2^-70).
+// Units: 2^-56 of the scale (pairs), 2^-70 (FP64, rounded from the threads' 2^-78: with 152
+// CTAs of 512 threads a total of 2^-10 of the scale is off by less than 2^-51 of itself, as
+// little as a sum in FP64 leaves; with units of 2^-62 it was 2^-44).
 constexpr long long kHighBias = 1ll << 39;
 constexpr long long kLowMask = (1ll << 40) - 1;
 template <bool MIXED>
@@ -165,12 +167,12 @@ LF_FIXED bool fp64_total(int e, unsigned long long low, unsigned long long high,
     word_parts(low, high, n, lo, hi);
     hi += lo >> 40;
     lo &= kLowMask;
-    const bool ok = hi >= (1ll << 12) && hi < (1ll << 45);
-    const int lead = fx_clz(hi);  // 19 to 51
+    const bool ok = hi >= (1ll << 20) && hi < (1ll << 45);  // units of 2^-30
+    const int lead = fx_clz(hi);  // 19 to 43
     const unsigned long long w = (static_cast<unsigned long long>(hi) << lead) |
                                  ((static_cast<unsigned long long>(lo) << 24) >> ((64 - lead) & 63));
     const unsigned long long m = (w >> 11) + ((w >> 10) & 1);  // 53 bits, rounded
-    out = fx_double(static_cast<long long>(static_cast<unsigned long long>(1023 + 41 - lead + e - 1) << 52) +
+    out = fx_double(static_cast<long long>(static_cast<unsigned long long>(1023 + 33 - lead + e - 1) << 52) +
                     static_cast<long long>(m));
     return ok;
 }

@@ -27,7 +27,7 @@
 // a CTA in shared memory; a CTA's sum then travels in two words, added to two
 // counters in L2 by red.add.  The top byte of a word counts the arrivals, so the poll
 // that sees the last CTA also has the sum.  Integers: the order of arrival does not
-// matter, and the total is that of the shares to 2^-56 (FP32 pairs) or 2^-62 (FP64) of
+// matter, and the total is that of the shares to 2^-56 (FP32 pairs) or 2^-70 (FP64) of
 // the scale.  A share out of range, or a total that lost more than ten bits of the
 // scale, sends all CTAs to a plain sum of FP64 totals behind a counter.  A crossing of
 // 152 CTAs takes 0.83 us this way (1.40 us with a release and acquire that publish z),

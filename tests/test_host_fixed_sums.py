@@ -2,9 +2,10 @@
 a total that is accepted is the exact sum of the shares to the sums' units, whatever the
 shares, and one near the last total is accepted.
 
-Bounds, with the scale 2^e <= the last total: a share, an FP32 pair, is rounded to 2^-56
-of the scale, by half a unit and a quarter more for the remainders' own sum; the total,
-a pair, to 2^-46 of itself.
+Bounds, with the scale 2^e <= the last total: a share is rounded to 2^-56 (FP32 pairs)
+or 2^-78 (FP64) of the scale, a CTA's FP64 sum to 2^-70, each by half a unit (pairs: a
+quarter more for the remainders' own sum); the total to 2^-46 (a pair) or 2^-53 of
+itself.
 """
 
 import math
@@ -54,7 +55,10 @@ def check(sums, cases):
         exact = math.fsum(values.ravel())
         scale = 2.0 ** math.floor(math.log2(previous))
         if accepted:
-            bound = shares.size * 1.25 * 2.0 ** -57 * scale + 2.0 ** -46 * abs(exact)
+            units = 1.25 * 2.0 ** -57 if mixed else 2.0 ** -79
+            bound = shares.size * units * scale + 2.0 ** (-46 if mixed else -53) * abs(exact)
+            if not mixed:
+                bound += shares.shape[0] * 2.0 ** -71 * scale
             assert abs(hi + lo - exact) <= bound, (mixed, shares.shape, exact / scale)
         else:
             assert not (2.0 ** -9 <= exact / scale <= 8.0 and np.abs(shares).max() < 8 * scale), (shares.shape,
@@ -62,7 +66,7 @@ def check(sums, cases):
     return results[:, 0]
 
 
-@pytest.mark.parametrize("mixed", [True])
+@pytest.mark.parametrize("mixed", [True, False])
 def test_random_shares(sums, mixed):
     """Totals from 2^-14 to 2^14 of the last one, shares of one size and of many."""
     rng = np.random.default_rng(7)
@@ -79,7 +83,7 @@ def test_random_shares(sums, mixed):
     assert 0.3 < accepted.mean() < 0.9  # both ways are met
 
 
-@pytest.mark.parametrize("mixed", [True])
+@pytest.mark.parametrize("mixed", [True, False])
 def test_equal_shares_up_to_their_limit(sums, mixed):
     """Every thread's share the same, from far below the last total to the largest share a
     thread may have: sums that run past a limb, a word or 64 bits are not taken for small
