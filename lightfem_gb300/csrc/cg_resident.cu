@@ -1412,7 +1412,7 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
 }
 
 bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms) {
-    if (!c.paired || c.num_sms > 255 || c.n < 2) return false;
+    if (!c.paired || c.num_sms >= 255 || c.n < 2) return false;  // a word counts arrivals in a byte (answered())
     const bool mixed = s.mixed != 0;
     Shape sh;
     if (!resident_structure(c, mixed, sh)) return false;
