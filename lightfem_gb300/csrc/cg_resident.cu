@@ -1411,10 +1411,11 @@ static bool resident_structure(Context& c, bool mixed, Shape& s) {
     return true;
 }
 
-bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms) {
+// Everything a solve needs on the device, and the kernel's arguments; false when the
+// resident kernel does not take the pattern.
+static bool resident_setup(Context& c, const SolveSetup& s, Shape& sh, ResArgs& a) {
     if (!c.paired || c.num_sms >= 255 || c.n < 2) return false;  // a word counts arrivals in a byte (answered())
     const bool mixed = s.mixed != 0;
-    Shape sh;
     if (!resident_structure(c, mixed, sh)) return false;
     Context::Resident& res = c.resident;
     const int nb = static_cast<int>(c.n / 2), slices = slices_of(c);
@@ -1438,7 +1439,6 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
         c.launches += 1;
         res.k_version[mixed] = c.k_version;
     }
-    ResArgs a{};
     a.nb = nb;
     a.slices = slices;
     a.grid = sh.grid;
@@ -1508,6 +1508,21 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
     a.maxit = s.max_iterations;
     a.max_ref = s.max_refinements;
     a.restart = s.restart;
+    return true;
+}
+
+bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms) {
+    Shape sh;
+    ResArgs a{};
+    try {
+        if (!resident_setup(c, s, sh, a)) return false;
+    } catch (const Error& e) {
+        if (e.code != LFGPU_ERR_NOMEM) throw;
+        // No room for the slices beside K: the graph of kernels reads K as it is.
+        c.resident.release();
+        return false;
+    }
+    const bool mixed = s.mixed != 0, jac = s.precond == LFGPU_PRECOND_JACOBI;
     auto launch = [&](auto kernel) {
         allow_dynamic_smem(kernel);
         if (sh.sync == kCluster && sh.grid > 8)

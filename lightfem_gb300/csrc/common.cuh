@@ -63,7 +63,13 @@ struct Buf {
         if (n == 0) return;
         // Round up to 64 elements so vectorised tails never leave the allocation.
         const size_t padded = (n + 63) / 64 * 64;
-        LF_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), padded * sizeof(T)));
+        const cudaError_t err = cudaMalloc(reinterpret_cast<void**>(&p), padded * sizeof(T));
+        if (err != cudaSuccess) {
+            cudaGetLastError();  // else the next launch would report it
+            p = nullptr;
+            throw Error{err == cudaErrorMemoryAllocation ? LFGPU_ERR_NOMEM : LFGPU_ERR_CUDA,
+                        "cudaMalloc of " + std::to_string(padded * sizeof(T)) + " bytes: " + cudaGetErrorString(err)};
+        }
         count = n;
     }
     void release() {
@@ -235,6 +241,23 @@ struct Context {
         Buf<unsigned long long> words;   // packed sums
         Buf<unsigned long long> tagged;  // z as tagged words
         unsigned long long pattern_version = ~0ull, k_version[2] = {~0ull, ~0ull};
+        void release() {
+            for (Grid& g : grid) {
+                g.window.release();
+                g.version = ~0ull;
+            }
+            group_ptr.release();
+            info.release();
+            off.release();
+            v32.release();
+            d32.release();
+            dlo.release();
+            v64.release();
+            d64.release();
+            words.release();
+            tagged.release();
+            pattern_version = k_version[0] = k_version[1] = ~0ull;
+        }
     } resident;
     bool resident_ran = false;  // the last solve ran there
 

@@ -1,0 +1,22 @@
+/* Preloaded where the CUDA runtime is the shared library LIBCUDART: the k-th cudaMalloc from now on finds no memory
+ * (it asks the driver for 2^50 bytes, so that the error is a real one in every respect). */
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+
+static long countdown = 0;
+
+void fail_allocation(long k) { countdown = k; }
+long allocations_to_go(void) { return countdown; }
+
+int cudaMalloc(void** p, size_t n) {
+    static int (*real)(void**, size_t) = 0;
+    if (!real) {
+        /* The runtime came in with a library opened locally: it is in no scope that RTLD_NEXT sees. */
+        void* runtime = dlopen(LIBCUDART, RTLD_LAZY | RTLD_NOLOAD);
+        if (runtime) real = (int (*)(void**, size_t))dlsym(runtime, "cudaMalloc");
+        if (!real) return 999; /* cudaErrorUnknown */
+    }
+    if (countdown > 0 && --countdown == 0) n = (size_t)1 << 50;
+    return real(p, n);
+}
