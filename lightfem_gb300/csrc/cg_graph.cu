@@ -108,7 +108,6 @@ struct CgArgs {
     const int* sub_begin;
     const long long* sub_fac;      // packed lower factor offset of each subdomain
     const double* sub_factor;      // by rows
-    const double* sub_factor_t;    // by columns
     const float* sub_inv32;        // mixed loop: block inverses, FP32 D x D squares
     const long long* sub_sq;       // offset of each subdomain's square
     // IC(0) level-scheduled sweeps (ic0.cu builds the schedules): [0] forward, [1] backward
@@ -1840,12 +1839,15 @@ __global__ void __launch_bounds__(kThreads) ic0_dot(CgArgs a) {
 // memory (a bounded poll of the value itself), then works its own unknowns out by
 // shuffles; no barrier holds the warp with the chain, and no warp issues terms it has
 // no rows for.  CTAs that share an SM start on different quarters, the largest
-// subdomains start first.  The factor's entries come a group or two ahead, a warp's 32
-// rows from consecutive addresses: forward from the copy by columns, backward from the
-// rows.  us an application, before (a barrier an unknown, predicated terms, both sweeps
-// along rows) and now, GB300, 64-node RCB blocks (up to 256 DOFs): 20x20, 7 blocks, 135
-// and 80 (the chain: 350 cycles an unknown); 180x160, 456 blocks, 300 and 102; 400x400,
-// 2513 blocks, 646 and 300 (the FP64 pipe), 1000x1000 5650 and 1711; 16-node blocks at 180x160 58 and 39.
+// subdomains start first.  The factor's entries come a group or two ahead: forward, a
+// lane's four of a group from its own row, a sector or two; backward, a warp's 32 of a row from
+// consecutive addresses.  (With a second copy of the factor by columns, so that the forward
+// sweep's were consecutive too: no faster anywhere, 103 us at 180x160, 129 with 100-node
+// blocks and 1281 at 400x400 with 250-node blocks, where the rows take 102, 114 and 1242.)
+// us an application, before (a barrier an unknown, predicated terms) and now, GB300, 64-node
+// RCB blocks (up to 256 DOFs): 20x20, 7 blocks, 135 and 80 (the chain: 350 cycles an
+// unknown); 180x160, 456 blocks, 300 and 102; 400x400, 2513 blocks, 646 and 296 (the FP64
+// pipe), 1000x1000 5650 and 1708; 16-node blocks at 180x160 58 and 38.
 // Publishing a group at a time instead of each unknown: 84, 105 and 307.
 constexpr int kSubGroup = 4;
 // poll_shared where the value comes from another warp: no back-off.
@@ -1870,7 +1872,6 @@ __global__ void __launch_bounds__(LFGPU_SUBDOMAIN_MAX_DOFS) subdomain_apply(CgAr
     const int begin = a.sub_begin[s], D = a.sub_begin[s + 1] - begin;
     if (first >= D) return;
     const double* __restrict__ by_row = a.sub_factor + a.sub_fac[s];
-    const double* __restrict__ by_col = a.sub_factor_t + a.sub_fac[s];
     const bool mine = i < D;
     const int dof = mine ? a.sub_dofs[begin + i] : 0;
     const double inv = mine ? __ldg(by_row + i * (i + 1) / 2 + i) : 0.0;
@@ -1879,13 +1880,13 @@ __global__ void __launch_bounds__(LFGPU_SUBDOMAIN_MAX_DOFS) subdomain_apply(CgAr
     double acc = mine ? a.r[dof] : 0.0, x = 0.0, c0[kSubGroup], c1[kSubGroup];
 
     // Forward: entries (i, j) below the diagonal, j ascending.
-    int j = 0, at = i;
+    int j = 0, at = i * (i + 1) / 2;
     const int below = mine ? i : 0;
     auto columns = [&](double* c) {
 #pragma unroll
         for (int u = 0; u < kSubGroup; ++u) {
-            c[u] = j < below ? __ldg(by_col + at) : 0.0;
-            at += D - 1 - j++;  // column j + 1 starts at its diagonal
+            c[u] = j++ < below ? __ldg(by_row + at) : 0.0;
+            ++at;
         }
     };
     auto subtract_y = [&](const double* c, int j0) {
@@ -2617,7 +2618,6 @@ SeparateApply subdomain_args(Context& c, CgArgs& a) {
     a.sub_begin = c.sub_begin;
     a.sub_fac = c.sub_fac_begin;
     a.sub_factor = c.sub_factor;
-    a.sub_factor_t = c.sub_factor_t;
     a.sub_inv32 = c.sub_inv32;
     a.sub_sq = c.sub_sq_begin;
     SeparateApply ap{};

@@ -281,7 +281,7 @@ struct Context {
     Buf<int> sub_dofs, sub_begin, sub_owner, sub_local;  // DOFs by subdomain; per DOF: subdomain, slot
     Buf<int> sub_order;           // the subdomains, largest first
     Buf<long long> sub_fac_begin;
-    Buf<double> sub_factor, sub_factor_t;  // packed lower triangles by rows, and by columns
+    Buf<double> sub_factor;       // packed lower triangles by rows
     Buf<float> sub_inv32;     // mixed loop: each block's inverse, D x D in FP32 (per K version)
     Buf<long long> sub_sq_begin;  // offsets of D x D scratch per subdomain (the inverse's FP64 work)
     unsigned long long sub_inv_version = ~0ull;

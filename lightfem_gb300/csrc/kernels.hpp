@@ -55,12 +55,6 @@ PcgResult run_pcg_separate(Context& c, const SolveSetup& s, float* kernel_ms, do
 // One FP64 application z = M^-1 r of the built preconditioner, on the stream.
 void launch_precond_apply(Context& c, int precond, const double* r, double* z);
 
-// Start of column j of a packed lower triangle of dimension d kept by columns.
-#ifdef __CUDACC__
-__host__ __device__
-#endif
-inline int subdomain_column(int d, int j) { return j * d - j * (j - 1) / 2; }
-
 // subdomain.cu: subdomain block-Jacobi split (per mesh and setting) and factor
 // (per K version)
 void ensure_subdomains(Context& c);

@@ -14,8 +14,7 @@
 // rounded on its own.  So the factor equals the reference's bit for bit.  A block
 // whose pivot is not positive and finite becomes the identity, as there.  The
 // packed lower factor stores reciprocal pivots on its diagonal, as the
-// reference's does.  It is kept twice, by rows and by columns, so that both sweeps of
-// an application read consecutive entries across a warp.
+// reference's does.
 //
 // For the mixed loop the setup also builds each block's inverse from the FP64
 // factor and stores it in FP32 as a full square (ensure_subdomain_inverse).
@@ -36,7 +35,7 @@ __global__ void __launch_bounds__(LFGPU_SUBDOMAIN_MAX_DOFS) subdomain_factor_ker
     const int* __restrict__ rowptr, const int* __restrict__ col, const double* __restrict__ K,
     const int* __restrict__ sub_dofs, const int* __restrict__ sub_begin, const int* __restrict__ owner,
     const int* __restrict__ local, const long long* __restrict__ fac_begin, double* factor,
-    double* __restrict__ factor_t, unsigned long long* __restrict__ degenerate) {
+    unsigned long long* __restrict__ degenerate) {
     __shared__ double colj[LFGPU_SUBDOMAIN_MAX_DOFS];  // column j of L below the pivot
     __shared__ int s_fail;
     const int s = blockIdx.x;
@@ -96,13 +95,6 @@ __global__ void __launch_bounds__(LFGPU_SUBDOMAIN_MAX_DOFS) subdomain_factor_ker
         }
     }
     if (fail && t == 0) atomicAdd(degenerate, 1ull);
-    __syncthreads();
-    // The same triangle by columns, for the application's forward sweep.
-    double* Lt = factor_t + fac_begin[s];
-    for (int i = warp; i < D; i += W) {
-        const double* ri = row(i);
-        for (int m = lane; m <= i; m += 32) Lt[subdomain_column(D, m) + (i - m)] = ri[m];
-    }
 }
 
 // subdomain_capture_ratio (src/precond.cpp:107-119): entries whose row and column
@@ -246,7 +238,6 @@ void ensure_subdomains(Context& c) {
         build_split(c);
     if (c.sub_k_version == c.k_version) return;
     c.sub_factor.ensure(static_cast<size_t>(std::max<long long>(1, c.sub_factor_size)));
-    c.sub_factor_t.ensure(static_cast<size_t>(std::max<long long>(1, c.sub_factor_size)));
     c.scratch64.ensure(64);
     unsigned long long* counters = reinterpret_cast<unsigned long long*>(c.scratch64.p + 24);  // degenerate, inside
     LF_CUDA(cudaMemsetAsync(counters, 0, 2 * sizeof(unsigned long long), c.stream));
@@ -254,7 +245,7 @@ void ensure_subdomains(Context& c) {
     if (c.sub_count > 0)
         subdomain_factor_kernel<<<static_cast<unsigned>(c.sub_count), threads, 0, c.stream>>>(
             c.rowptr, c.col, c.K, c.sub_dofs, c.sub_begin, c.sub_owner, c.sub_local, c.sub_fac_begin, c.sub_factor,
-            c.sub_factor_t, counters);
+            counters);
     subdomain_capture_kernel<<<grid_for(c.n, kCaptureThreads, 16 * c.num_sms), kCaptureThreads, 0, c.stream>>>(
         static_cast<int>(c.n), c.rowptr, c.col, c.sub_owner, counters + 1);
     c.launches += c.sub_count > 0 ? 2 : 1;

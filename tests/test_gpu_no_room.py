@@ -1,7 +1,8 @@
 """A solve whose second copy of the matrix finds no device memory: it runs as the graph of
 kernels, which reads the matrix as it is, and the handle goes back to the resident kernel
 once there is room.  Every allocation of a first solve fails in turn, by a cudaMalloc
-preloaded in a process of its own (tests/host/failing_malloc.c)."""
+preloaded in a process of its own (tests/host/failing_malloc.c), which also tells what
+the subdomain blocks ask for."""
 
 import glob
 import json
@@ -62,6 +63,29 @@ print(json.dumps(ends))
 """
 
 
+MEMORY = r"""
+import ctypes, json, sys
+import numpy as np
+sys.path[:0] = [sys.argv[1], sys.argv[1] + "/tests"]
+from cases import indexed
+from lightfem_gb300 import _native as native, mesh
+from lightfem_gb300.solver import upload_model
+
+fake = ctypes.CDLL(sys.argv[2])
+fake.bytes_asked.restype = ctypes.c_long
+model = indexed(mesh.cantilever(99, 101, per_element_young=mesh.lognormal_moduli(9999, seed=3)))
+owner, _ = native.host_subdomains(model.xy, 64)
+size = 2 * np.bincount(owner)
+ctx = native.Context(0)
+upload_model(ctx, model)
+ctx.assemble("coloring")
+ctx.apply_dirichlet()
+before = fake.bytes_asked()
+ctx.solve(ctx.options(1e-10, 20000, "csr", "subdomain"))
+print(json.dumps([fake.bytes_asked() - before, int((size * (size + 1) // 2).sum()) * 8]))
+"""
+
+
 @pytest.fixture(scope="module")
 def ends_of(native, tmp_path_factory):
     from lightfem_gb300 import build
@@ -75,8 +99,8 @@ def ends_of(native, tmp_path_factory):
     subprocess.run([os.environ.get("CC", "gcc"), "-shared", "-fPIC", "-O1", f'-DLIBCUDART="{cudart}"',
                     os.path.join(ROOT, "tests", "host", "failing_malloc.c"), "-o", fake, "-ldl"], check=True)
 
-    def run(precond, precision):
-        r = subprocess.run([sys.executable, "-c", SCRIPT, ROOT, fake, precond, precision], capture_output=True,
+    def run(*args, script=SCRIPT):
+        r = subprocess.run([sys.executable, "-c", script, ROOT, fake, *args], capture_output=True,
                            text=True, timeout=300, env={**os.environ, "LD_PRELOAD": fake, "LFGPU_LIBRARY": lib})
         assert r.returncode == 0, r.stderr[-2000:]
         return json.loads(r.stdout.splitlines()[-1])
@@ -93,3 +117,9 @@ def test_slices(native, ends_of, precision):
     assert len(graph) >= 5 and all(e["launches"] > e["iterations"] for e in graph), ends
     # 1e-10 of the residual at both ends: the repository's bar for displacements
     assert all(e["converged"] and e["off"] <= 1e-8 for e in graph), ends
+
+
+def test_subdomain_factor_is_kept_once(ends_of):
+    asked, factor = ends_of(script=MEMORY)
+    # the vectors and the split take a quarter of the factor here, not another factor
+    assert factor <= asked < 1.5 * factor
