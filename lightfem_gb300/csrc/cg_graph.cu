@@ -2269,6 +2269,7 @@ void add_kernel(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraphNode_t* dep
 struct StagedShape {
     int grid, smem, stash;
 };
+constexpr int kStagedStaticSmem = 4096;
 template <int PRECOND>
 StagedShape staged_shape(int nb) {
     int dev = 0, sms = 0, smem_sm = 0, per_sm = 0;
@@ -2276,11 +2277,11 @@ StagedShape staged_shape(int nb) {
     LF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     LF_CUDA(cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
     const int stages = kStagedStages * staged_stage_bytes<PRECOND>();
-    const int share = smem_sm / kStagedCtasPerSm - 4096;  // less the static arrays and the per-CTA reservation
+    const int share = smem_sm / kStagedCtasPerSm - kStagedStaticSmem;  // which covers the per-CTA reservation too
     const int grid = kStagedCtasPerSm * sms;
     const int stash = std::max(0, std::min((share - stages) / 16, staged_per_cta(nb, grid)));
     StagedShape sh{grid, stages + 16 * stash, stash};
-    allow_dynamic_smem(mx_update_staged<PRECOND>);
+    allow_dynamic_smem(mx_update_staged<PRECOND>, kStagedStaticSmem);
     LF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mx_update_staged<PRECOND>, kStagedBlock, sh.smem));
     LF_REQUIRE(per_sm >= 1, LFGPU_ERR_CUDA, "the staged update does not fit an SM");
     sh.grid = std::min(grid, per_sm * sms);
@@ -2665,13 +2666,13 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         a.sw_rr = c.sweep_rr32.p;
         if (piped) {
             ap.smem = pipe.smem;
-            allow_dynamic_smem(ic0_pipe_sweep<2>);
-            allow_dynamic_smem(ic0_pipe_sweep<3>);
+            allow_dynamic_smem(ic0_pipe_sweep<2>, kSweepStaticSmem);
+            allow_dynamic_smem(ic0_pipe_sweep<3>, kSweepStaticSmem);
             return ap;
         }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(float)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
-        allow_dynamic_smem(ic0_level_sweep<2>);
-        allow_dynamic_smem(ic0_level_sweep<3>);
+        allow_dynamic_smem(ic0_level_sweep<2>, kSweepStaticSmem);
+        allow_dynamic_smem(ic0_level_sweep<3>, kSweepStaticSmem);
     } else {
         c.sweep_y.ensure(c.n + kSweepSlack);
         c.sweep_rhs.ensure(c.n + kSweepSlack);
@@ -2679,13 +2680,13 @@ SeparateApply sweep_args(Context& c, CgArgs& a, bool fp32) {
         a.sw_rhs = c.sweep_rhs.p;
         if (piped) {
             ap.smem = pipe.smem;
-            allow_dynamic_smem(ic0_pipe_sweep<0>);
-            allow_dynamic_smem(ic0_pipe_sweep<1>);
+            allow_dynamic_smem(ic0_pipe_sweep<0>, kSweepStaticSmem);
+            allow_dynamic_smem(ic0_pipe_sweep<1>, kSweepStaticSmem);
             return ap;
         }
         ap.smem = sweep_smem_bytes(static_cast<int>(sizeof(double)), c.sweep_window, c.sweep_maxp, c.sweep_maxe);
-        allow_dynamic_smem(ic0_level_sweep<0>);
-        allow_dynamic_smem(ic0_level_sweep<1>);
+        allow_dynamic_smem(ic0_level_sweep<0>, kSweepStaticSmem);
+        allow_dynamic_smem(ic0_level_sweep<1>, kSweepStaticSmem);
     }
     return ap;
 }

@@ -1524,7 +1524,7 @@ bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel
     }
     const bool mixed = s.mixed != 0, jac = s.precond == LFGPU_PRECOND_JACOBI;
     auto launch = [&](auto kernel) {
-        allow_dynamic_smem(kernel);
+        allow_dynamic_smem(kernel, s.mixed ? kStaticSmem32 : kStaticSmem64);
         if (sh.sync == kCluster && sh.grid > 8)
             LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         cudaLaunchConfig_t cfg = {};

@@ -34,18 +34,16 @@ struct Error {
         if (!(cond)) throw ::lfgpu::Error{(code), (msg)}; \
     } while (0)
 
-// Lets a kernel be launched with any dynamic shared memory a CTA can have.  The limit is
-// an attribute of the kernel, shared by all handles and threads: every call sets the same
-// value, so that none lowers it between another's call and launch.
+// Lets a kernel be launched with any dynamic shared memory a CTA can have beside
+// static_bytes (at least its static shared memory).  The limit is an attribute of the
+// kernel, shared by all handles and threads: every call sets the same value, so that none
+// lowers it between another's call and launch.
 template <typename K>
-void allow_dynamic_smem(K kernel) {
+void allow_dynamic_smem(K kernel, int static_bytes) {
     int device = 0, optin = 0;
-    cudaFuncAttributes attr{};
     LF_CUDA(cudaGetDevice(&device));
     LF_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    LF_CUDA(cudaFuncGetAttributes(&attr, kernel));
-    LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 optin - static_cast<int>(attr.sharedSizeBytes)));
+    LF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - static_bytes));
 }
 
 // Device buffer that grows on demand and is released with its owner (the handle).
