@@ -83,8 +83,9 @@ enum {
     LFGPU_OPTION_IC0_SWEEP = 1      /* LFGPU_IC0_SWEEP_*: how the IC(0) triangular sweeps are scheduled */
 };
 /* AUTO: by levels in one thread block, several levels at once, when no dependency
- * level holds more than 256 rows and the schedule fits its shared memory; else by
- * levels as LEVELS when they hold 192 rows or more on average and fit; else POLLED.
+ * level holds more than 256 rows and the schedule fits both its shared memory and the
+ * ring that LEVELS uses; else by levels as LEVELS when they hold 192 rows or more on
+ * average and fit; else POLLED.
  * The mixed-precision loop always sweeps by levels.
  * LEVELS: one thread-block cluster walks the levels, LFGPU_ERR_UNSUPPORTED where the
  * schedule does not fit the cluster's shared-memory ring.
@@ -112,8 +113,8 @@ typedef struct lfgpu_solve_options {
     int64_t max_refinements;   /* mixed: cap on FP64 residual replacements */
     int32_t persistent;        /* 1: the persistent kernel with TMA-staged products; 0: one resident kernel
                                   for Jacobi and 2x2 blocks, where the pattern is paired and its rows'
-                                  columns fit a window in shared memory, else a device-driven CUDA graph of
-                                  per-phase kernels (conditional WHILE node) */
+                                  columns fit a window in shared memory and a second copy of K the device,
+                                  else a device-driven CUDA graph of per-phase kernels (conditional WHILE node) */
     int32_t unrolled;          /* profiling only, graph loop: > 0 replaces the conditional loop by a plain
                                   graph of this many iterations (profilers do not descend into
                                   conditional bodies); the solve stops there */

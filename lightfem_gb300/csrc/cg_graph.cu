@@ -1,7 +1,7 @@
 // Preconditioned CG as a device-driven CUDA graph: the separately applied
 // preconditioners, the profiling form, and the pointwise preconditioners where the
 // resident kernel (cg_resident.cu) does not take the pattern (unpaired, or rows whose
-// columns span more nodes than a CTA's shared memory holds).
+// columns span more nodes than a CTA's shared memory holds) or finds no room for its copy.
 //
 // Same recurrences as the persistent kernel in pcg.cu (pcg_solve,
 // src/solver.cpp:532-627, in FP64; the FP32-inner / FP64-refinement scheme in

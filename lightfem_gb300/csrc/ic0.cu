@@ -377,7 +377,8 @@ bool ic0_use_pipe(const Context& c, bool fp32) {
 }
 
 // LFGPU_IC0_SWEEP_AUTO takes the pipelined sweeps where no level is wider than
-// kPipeMaxWidth rows and the schedule fits one CTA.  Per forward + backward application
+// kPipeMaxWidth rows and the schedule fits one CTA and the cluster's ring (a schedule that
+// the ring refuses stays refused by mixed solves).  Per forward + backward application
 // on GB300 (cantilevers, RCM; polled / levels / pipelined): 96x96, up to 49 rows a level,
 // 1.77 / 2.74 / 0.62 ms; 250x250, 126 rows: 5.24 / 7.11 / 2.29; 500x500, 251 rows:
 // 13.95 / 14.34 / 7.61; a mixed iteration there, levels / pipelined: 1.07 / 0.40,

@@ -43,7 +43,8 @@ struct SolveSetup {
 PcgResult run_pcg(Context& c, const SolveSetup& s, float* kernel_ms);
 
 // cg_resident.cu: the same solver for the pointwise preconditioners in one resident
-// kernel; false (nothing done) when the pattern is not one it takes
+// kernel; false (nothing solved) when the pattern is not one it takes or its copy of the
+// matrix finds no device memory
 bool run_resident(Context& c, const SolveSetup& s, PcgResult* out, float* kernel_ms);
 
 // cg_graph.cu: the same solver as a device-driven CUDA graph of per-phase kernels
