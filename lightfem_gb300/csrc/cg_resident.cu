@@ -633,24 +633,60 @@ __device__ __forceinline__ double2 slice_row(const ResArgs& a, int s, int node, 
 }
 
 // (f - K x) of one node in FP64 from the CSR values of a paired pattern (rows 2i and
-// 2i + 1 share their columns); x as other CTAs wrote it.
+// 2i + 1 share their columns); x as other CTAs wrote it.  A row's terms go to four sums by
+// their place modulo four, as in the CSR product: those with u and those with v cancel
+// apart from one another, and in one sum they leave a residual whose rounding is up to
+// twice as large.  It bounds what a mixed solve can reach: of 800 solves at
+// tolerances of 1e-9 to 1e-12 with moduli over four decades 363 converged within 20,000
+// iterations with one sum a row, 408 with four, 404 in the graph of kernels.  WIDE:
+// both rows and all sums at once; else, with 64 registers a thread, a row and two sums at a
+// time (all at once spills, and costs the loop around it 4 to 14 %).
+template <bool WIDE>
 __device__ __forceinline__ double2 residual_row(const ResArgs& a, int node, const double* x) {
     const int b = __ldg(a.rowptr + 2 * node), len = __ldg(a.rowptr + 2 * node + 1) - b;
     const double2* k0 = reinterpret_cast<const double2*>(a.K + b);
-    const double2* k1 = reinterpret_cast<const double2*>(a.K + b + len);
-    double s0 = 0.0, s1 = 0.0;
     const int m = len / 2;
-#pragma unroll 3
-    for (int k = 0; k < m; ++k) {
-        const double2 xv = __ldcg(reinterpret_cast<const double2*>(x + __ldg(a.col + b + 2 * k)));
-        const double2 u = __ldg(k0 + k), w = __ldg(k1 + k);
-        s0 = fma(u.x, xv.x, s0);
-        s0 = fma(u.y, xv.y, s0);
-        s1 = fma(w.x, xv.x, s1);
-        s1 = fma(w.y, xv.y, s1);
+    double sum[2] = {0.0, 0.0};
+    if constexpr (WIDE) {
+        const double2* k1 = reinterpret_cast<const double2*>(a.K + b + len);
+        double s0[4] = {}, s1[4] = {};
+#pragma unroll 1
+        for (int k = 0; k < m; k += 2) {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (k + j >= m) break;
+                const double2 xv = __ldcg(reinterpret_cast<const double2*>(x + __ldg(a.col + b + 2 * (k + j))));
+                const double2 u = __ldg(k0 + k + j), w = __ldg(k1 + k + j);
+                s0[2 * j] = fma(u.x, xv.x, s0[2 * j]);
+                s0[2 * j + 1] = fma(u.y, xv.y, s0[2 * j + 1]);
+                s1[2 * j] = fma(w.x, xv.x, s1[2 * j]);
+                s1[2 * j + 1] = fma(w.y, xv.y, s1[2 * j + 1]);
+            }
+        }
+        sum[0] = (s0[0] + s0[1]) + (s0[2] + s0[3]);
+        sum[1] = (s1[0] + s1[1]) + (s1[2] + s1[3]);
+    } else {
+#pragma unroll 2
+        for (int row = 0; row < 2; ++row) {
+            double t = 0.0;
+#pragma unroll 1
+            for (int j = 0; j < 2; ++j) {
+                double su = 0.0, sv = 0.0;
+#pragma unroll 1
+                for (int k = j; k < m; k += 2) {
+                    const double2 xv = __ldcg(reinterpret_cast<const double2*>(x + __ldg(a.col + b + 2 * k)));
+                    const double2 u = __ldg(k0 + row * m + k);
+                    su = fma(u.x, xv.x, su);
+                    sv = fma(u.y, xv.y, sv);
+                }
+                t += su + sv;
+            }
+            if (row) sum[1] = t;
+            else sum[0] = t;
+        }
     }
     const double2 fv = __ldg(reinterpret_cast<const double2*>(a.f) + node);
-    return make_double2(fv.x - s0, fv.y - s1);
+    return make_double2(fv.x - sum[0], fv.y - sum[1]);
 }
 
 template <int PRECOND>
@@ -722,6 +758,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
     using Sum = typename std::conditional<MIXED, FloatPair, double>::type;
     using Tot = Total<MIXED>;
     constexpr bool kPublish = SYNC == kPublished;
+    constexpr bool kWide = max_threads(MIXED, CACHED) < 1024;
     static_assert(max_threads(MIXED, CACHED) <= kLimbThreads<MIXED>, "the CTA's limb sums would overflow");
     extern __shared__ __align__(16) unsigned char res_smem[];
     __shared__ ResShared sh;
@@ -862,7 +899,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
             double2 xv = make_double2(0.0, 0.0), rv;
             if (a.x0) {
                 xv = reinterpret_cast<const double2*>(a.x0)[node];
-                rv = residual_row(a, node, a.x0);
+                rv = residual_row<kWide>(a, node, a.x0);
             } else {
                 rv = __ldg(reinterpret_cast<const double2*>(a.f) + node);
             }
@@ -1049,7 +1086,7 @@ __global__ void __launch_bounds__(max_threads(MIXED, CACHED), 1) resident_pcg(Re
             tag += 1;
             z_bar = 3;
             each_node([&](int, int node, int at) {
-                const double2 rv = residual_row(a, node, a.x);
+                const double2 rv = residual_row<kWide>(a, node, a.x);
                 const float2 rw = to_working(rv, float2{});
                 const float2 zv = precond_at<PRECOND>(a, node, rw);
                 publish(node, zv);

@@ -44,3 +44,40 @@ def test_replaced_residual_is_that_of_x(native, nx, ny):
         assert (r.iterations, r.refinements) == (rep.iterations, rep.refinements)
         np.testing.assert_array_equal(again, u)
     ctx.close()
+
+
+def summed(native, ctx, u, sums):
+    """||f - K u|| with a row's fused multiply-adds dealt to ``sums`` sums by their place."""
+    rp, col, _, _ = ctx.download_pattern()
+    k, f = ctx.download(native.K_CONSTRAINED), ctx.download(native.F_CONSTRAINED)
+    s = np.zeros((sums, ctx.n_dofs))
+    for e in range(np.diff(rp).max()):
+        live = np.diff(rp) > e
+        at = rp[:-1][live] + e
+        s[e % sums, live] = (np.longdouble(k[at]) * u[col[at]] + s[e % sums, live]).astype(np.float64)
+    return np.linalg.norm(f - (s[0] if sums == 1 else (s[0] + s[1]) + (s[2] + s[3])))
+
+
+# A cluster, and a grid whose threads have 64 registers
+@pytest.mark.parametrize("nx,ny,replacements", [(41, 37, range(11, 16)), (350, 350, (9, 11))])
+def test_residual_is_formed_in_four_sums(native, nx, ny, replacements):
+    """A replaced residual is that of the CSR product's four sums a row, and not that of
+    one sum, whose rounding is larger by up to a factor of two: it bounds what a mixed solve
+    can reach."""
+    ctx = native.Context(0)
+    upload_model(ctx, indexed(mesh.cantilever(
+        nx, ny, per_element_young=mesh.lognormal_moduli(nx * ny, seed=1, scale=70e9, sigma=2.0))))
+    ctx.assemble("coloring")
+    ctx.apply_dirichlet()
+    # The extended product rounds as an FMA does but for double rounding where long double
+    # has fewer than 106 bits.
+    tolerance = 1e-9 if np.finfo(np.longdouble).nmant >= 105 else 0.02
+    told = []
+    for precond in ("jacobi", "block"):
+        for count in replacements:
+            u, rep = ctx.solve(ctx.options(1e-15, 20000, "csr", precond, "mixed", max_refinements=count))
+            four, one = summed(native, ctx, u, 4), summed(native, ctx, u, 1)
+            told.append(abs(one - four) / four)
+            assert abs(rep.final_residual - four) <= tolerance * four
+    assert max(told) > 2 * tolerance  # the two can be told apart here
+    ctx.close()
