@@ -46,12 +46,11 @@
 //   FP64  graph  28.5        29.8        32.1  36.1  44.9  57.7        ~97         200
 //         here    4.8   4.9   5.6   6.0   7.2   8.5  13.7  20.3  29.4  45.2  68.1  103
 //   mixed graph  20.9        20.0        20.1  21.5  24.2  24.5   28   ~33         58
-//         here    2.3   2.6   2.7   3.1   4.1   4.3   5.1   7.1   7.9  11.3  21.8  33.7
+//         here    2.3   2.6   2.7   3.1   4.1   3.9   5.1   6.6   7.6  11.5  21.8  34.4
 // FP64 is bound by the FP64 pipe from 200 on (52 instructions a node; at 640 ncu counts it
-// busy for 79 % of the time, 36 us);
-// mixed by the crossings up to 400 and by HBM from 800 on, where K leaves L2.  With FP64
-// shuffles and FP64 scalars in the sums a mixed iteration took 3.9 us at 8, 6.0 at 50
-// and 7.6 at 200, an FP64 one 6.3, 7.8 and 11.2.
+// busy for 79 % of the time, 36 us); mixed by the crossings up to 400 and by HBM from 800
+// on, where K leaves L2.  With FP64 shuffles and FP64 scalars in the sums a mixed iteration
+// took 3.9 us at 8, 6.0 at 50 and 7.6 at 200, an FP64 one 6.3, 7.8 and 11.2.
 #include "cg_fixed.hpp"
 #include "cg_math.cuh"
 #include "common.cuh"
